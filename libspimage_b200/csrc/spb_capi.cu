@@ -92,6 +92,7 @@ int radix_plan(int n, int *radix) {
 
 struct Axis {
   LinePlan lp{};
+  MixPlan mix[2]{};  // consecutive short stages run as one where they can; every stage by itself
   float2 *tw = nullptr;
 };
 
@@ -117,11 +118,25 @@ int make_axis(Axis &ax, int n) {
     ns_ *= r;
   }
   if (st.empty()) st.push_back(make_float2(1.0f, 0.0f));
+  const size_t nst = st.size();
+  const bool mixed =
+      make_mix_plan(ax.mix[0], n, radix, ns, h.data(), true) && make_mix_plan(ax.mix[1], n, radix, ns, h.data(), false);
+  if (mixed)  // behind the stage tables: W_R^e of the prime steps (the same in both plans)
+    for (int i = 0; i < ax.mix[0].nsteps; i++) {
+      const MixStep &s = ax.mix[0].step[i];
+      if (!s.kind)
+        for (int e = 0; e < s.r; e++) st.push_back(h[(size_t)e * (n / s.r)]);
+    }
   CK(cudaMalloc(&ax.tw, sizeof(float2) * ((size_t)n + st.size())));
   CK(cudaMemcpy(ax.tw, h.data(), sizeof(float2) * (size_t)n, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(ax.tw + n, st.data(), sizeof(float2) * st.size(), cudaMemcpyHostToDevice));
   ax.lp.tw = ax.tw;
   ax.lp.stw = ax.tw + n;
+  for (MixPlan &mp : ax.mix) {
+    mp.stw = ax.lp.stw;
+    mp.pw = ax.lp.stw + nst;
+  }
+  ax.lp.mix = mixed ? ax.mix : nullptr;
   return 0;
 }
 
@@ -789,6 +804,11 @@ __global__ void build_amp_line_kernel(const float *amp, float *amp_line, int len
     if (!div_rn_nb_domain(v)) *bad = 1;
   }
 }
+// *bad as build_amp_line_kernel sets it, where no amplitude lines are built
+__global__ void check_amp_kernel(const float *amp, long long n, int *bad) {
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
+    if (!div_rn_nb_domain(amp[k])) *bad = 1;
+}
 // bit i of line L = measured flag of pixel i*estride + L (of start 0)
 __global__ void build_meas_bits_kernel(const uint8_t *flags, uint32_t *bits, int len, int W, long long estride,
                                        long long nlines) {
@@ -845,10 +865,14 @@ static int proj_geometry(spb_ctx *c) {
 }
 
 static int build_amp_line(spb_ctx *c) {
-  if (!proj_geometry(c)) return 0;
-  if (!c->amp_line) CK(cudaMalloc(&c->amp_line, sizeof(float) * (size_t)c->n));
   if (!c->amp_bad) CK(cudaMalloc(&c->amp_bad, sizeof(int)));
   CK(cudaMemsetAsync(c->amp_bad, 0, sizeof(int), c->st));
+  if (!proj_geometry(c)) {
+    check_amp_kernel<<<592, 256, 0, c->st>>>(c->amp, c->n, c->amp_bad);
+    CK(cudaGetLastError());
+    return 0;
+  }
+  if (!c->amp_line) CK(cudaMalloc(&c->amp_line, sizeof(float) * (size_t)c->n));
   build_amp_line_kernel<<<592, 256, 0, c->st>>>(c->amp, c->amp_line, c->proj_len, c->proj_estride, c->proj_lines,
                                                 c->amp_bad);
   CK(cudaGetLastError());

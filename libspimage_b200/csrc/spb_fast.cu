@@ -256,6 +256,8 @@ __global__ void __launch_bounds__(256) row_fast_kernel(PassArgs a, const float2 
         const float s = a.f32src[idx];
         x = make_float2(fmul(s, s), 0.0f);
       } else x = a.src[idx];
+      if constexpr (MODE == ROW_DM_F1_FWD)
+        if (!(a.flags[idx] & FLAG_INSIDE)) x = make_float2(fmul(-a.gamma1, x.x), fmul(-a.gamma1, x.y));
     }
     v[q] = x;
   }
@@ -267,7 +269,8 @@ __global__ void __launch_bounds__(256) row_fast_kernel(PassArgs a, const float2 
   }
   cp_async_wait_all();
   __syncthreads();
-  if constexpr (MODE == ROW_FWD || MODE == ROW_FWD_DEPHASE || MODE == ROW_FWD_F32 || MODE == ROW_FWD_SQUARE_F32) {
+  if constexpr (MODE == ROW_FWD || MODE == ROW_FWD_DEPHASE || MODE == ROW_FWD_F32 || MODE == ROW_FWD_SQUARE_F32 ||
+                MODE == ROW_DM_F1_FWD) {
     reg::fft<N, false>(v, line, t, tw_s);
     pdl_release();
     if (valid)
@@ -1312,6 +1315,7 @@ static cudaError_t row_fast_mode(int mode, const LinePlan &px, const PassArgs &a
     case ROW_INV_ABS: return row_fast_launch<N, ROW_INV_ABS>(px, a, st);
     case ROW_ITER: return row_fast_launch<N, ROW_ITER>(px, a, st);
     case ROW_DM_ITER: return row_fast_launch<N, ROW_DM_ITER>(px, a, st);
+    case ROW_DM_F1_FWD: return row_fast_launch<N, ROW_DM_F1_FWD>(px, a, st);
     case ROW_FWD_F32: return row_fast_launch<N, ROW_FWD_F32>(px, a, st);
     case ROW_FWD_SQUARE_F32: return row_fast_launch<N, ROW_FWD_SQUARE_F32>(px, a, st);
   }

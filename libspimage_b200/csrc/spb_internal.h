@@ -121,13 +121,47 @@ struct SelectState {
 };
 static_assert(sizeof(SelectState) == 8216, "the selection state keeps its size");
 
+// Steps of a line transform in the mixed-radix kernels (spb_mixed.cu): one
+// stage of the canonical plan, or two short consecutive ones run as one.
+// Radices with a kernel, and the pairs that have one; other radices (primes
+// from 7) are kind 0.  n * (the largest index a magic divides) stays below 2^32.
+#define SPB_MIX_KINDS(X) \
+  X(2, 1) X(3, 1) X(4, 1) X(5, 1) X(8, 1) X(16, 1) X(2, 3) X(2, 5) X(4, 3) X(3, 3) X(3, 5)
+__host__ __device__ constexpr int mix_kind(int r1, int r2) { return r1 * 32 + r2; }
+constexpr bool mix_single_ok(int r) { return r == 2 || r == 3 || r == 4 || r == 5 || r == 8 || r == 16; }
+constexpr bool mix_pair_ok(int r1, int r2) {
+  return (r1 == 2 && (r2 == 3 || r2 == 5)) || (r1 == 4 && r2 == 3) || (r1 == 3 && (r2 == 3 || r2 == 5));
+}
+constexpr int kMixMaxSteps = 9;
+constexpr size_t kMixSmem = 227 * 1024;  // dynamic shared memory a block may take
+struct MixStep {
+  int kind, r;              // r: points of a composite butterfly
+  int ns, nb;               // points between its outputs; butterflies per line (n / r)
+  unsigned ns_magic, nb_magic;  // quotients by ns and nb as a high product (unused for 1)
+  int tw1, tw2, pw;         // its tables: byte offsets in the stage table (first, second stage), entry of the prime tables
+  int din;                  // free elements after every ns points of its input
+  int sin, qout;            // elements between a butterfly's inputs, between the outputs of q and q + 1
+};
+struct MixPlan {
+  int n, nsteps, pitch;  // pitch: elements of a line's buffer
+  float neg0;            // -0 (see spb_mixed.cu)
+  const float2 *stw;     // stage tables (LinePlan::stw)
+  const float2 *pw;      // per prime step: W_R^e, e < R (device)
+  MixStep step[kMixMaxSteps];
+};
+// fills everything but the device pointers (pairs: run short consecutive
+// stages as one); false when the line has no plan here
+bool make_mix_plan(MixPlan &mp, int n, const int *radix, int nstages, const float2 *tw, bool pairs);
+cudaError_t launch_row_mixed(int mode, const LinePlan &px, const PassArgs &a, cudaStream_t st);
+cudaError_t launch_col_mixed(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st);
+
 // register-resident kernels (spb_fast.cu); cudaErrorNotSupported when the
 // line length or mode has none
 cudaError_t launch_row_fast(int mode, const LinePlan &px, const PassArgs &a, cudaStream_t st);
 cudaError_t launch_col_fast(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st);
 // whether the projection pass has a kernel of w columns per block for lines of n points
 bool col_width_ok(int n, int w);
-// the same for the general kernels' compile-time-plan lengths (192, 384, 1000)
+// the same for mixed-radix lines (192, 384 and 1000 points)
 bool general_col_width_ok(int n, int w);
 // all iterations of a call for every start of an N x N pattern (N = 32, 64,
 // 128), one block per start with its spectrum resident (spb_fast.cu); a.dst

@@ -19,10 +19,13 @@
 
 namespace spb {
 
+// The general passes below (run-time stage loops) serve lines of one point and
+// lines without a plan in the mixed-radix kernels (make_mix_plan); every other
+// line runs in spb_fast.cu, spb_split.cu or spb_mixed_*.cu.
+
 // ---------------------------------------------------------------- row pass
-template <int MODE, int NC>
-__device__ __forceinline__ void row_pass_body(const LinePlan &px, const PassArgs &a, int tpr, int rpb,
-                                              long long nrows) {
+template <int MODE>
+__global__ void __launch_bounds__(256) row_pass_kernel(LinePlan px, PassArgs a, int tpr, int rpb, long long nrows) {
   extern __shared__ float2 smem[];
   const int n = px.n;
   const int lr = threadIdx.x / tpr, t = threadIdx.x % tpr;
@@ -72,11 +75,11 @@ __device__ __forceinline__ void row_pass_body(const LinePlan &px, const PassArgs
 
   if constexpr (MODE == ROW_FWD || MODE == ROW_FWD_DEPHASE || MODE == ROW_FWD_F32 || MODE == ROW_FWD_SQUARE_F32 ||
                 MODE == ROW_DM_F1_FWD) {
-    float2 *r = line_fft_sel<false, NC>(A, B, px, 1, t, tpr, px.stw);
+    float2 *r = line_fft<false>(A, B, px, 1, t, tpr);
     if (valid)
       for (int i = t; i < n; i += tpr) a.dst[base + i] = r[i];
   } else if constexpr (MODE == ROW_INV || MODE == ROW_INV_SCALE || MODE == ROW_INV_ABS) {
-    float2 *r = line_fft_sel<true, NC>(A, B, px, 1, t, tpr, px.stw);
+    float2 *r = line_fft<true>(A, B, px, 1, t, tpr);
     if (valid) {
       for (int i = t; i < n; i += tpr) {
         if constexpr (MODE == ROW_INV) a.dst[base + i] = r[i];
@@ -87,7 +90,7 @@ __device__ __forceinline__ void row_pass_body(const LinePlan &px, const PassArgs
   } else if constexpr (MODE == ROW_ITER) {
     const float beta = iter_beta(a);
     const float one_m2b = fsub(1.0f, fmul(2.0f, beta));  // 1 - 2*beta in float, as the reference
-    float2 *r = line_fft_sel<true, NC>(A, B, px, 1, t, tpr, px.stw);
+    float2 *r = line_fft<true>(A, B, px, 1, t, tpr);
     for (int i = t; i < n; i += tpr) {
       float2 g = make_float2(0.0f, 0.0f);
       if (valid) {
@@ -112,13 +115,13 @@ __device__ __forceinline__ void row_pass_body(const LinePlan &px, const PassArgs
     }
     __syncthreads();
     float2 *o = (r == A) ? B : A;
-    float2 *x = line_fft_sel<false, NC>(r, o, px, 1, t, tpr, px.stw);
+    float2 *x = line_fft<false>(r, o, px, 1, t, tpr);
     if (valid)
       for (int i = t; i < n; i += tpr) a.dst[base + i] = x[i];
   } else if constexpr (MODE == ROW_DM_ITER) {
     const float beta = iter_beta(a);
-    float2 *rho = line_fft_sel<true, NC>(A, B, px, 1, t, tpr, px.stw);
-    float2 *fr = line_fft_sel<true, NC>(Cb, D, px, 1, t, tpr, px.stw);
+    float2 *rho = line_fft<true>(A, B, px, 1, t, tpr);
+    float2 *fr = line_fft<true>(Cb, D, px, 1, t, tpr);
     for (int i = t; i < n; i += tpr) {
       float2 g = make_float2(0.0f, 0.0f), f1 = g;
       if (valid) {
@@ -143,9 +146,9 @@ __device__ __forceinline__ void row_pass_body(const LinePlan &px, const PassArgs
     }
     __syncthreads();
     float2 *o1 = (rho == A) ? B : A;
-    float2 *x = line_fft_sel<false, NC>(rho, o1, px, 1, t, tpr, px.stw);
+    float2 *x = line_fft<false>(rho, o1, px, 1, t, tpr);
     float2 *o2 = (fr == Cb) ? D : Cb;
-    float2 *xf = line_fft_sel<false, NC>(fr, o2, px, 1, t, tpr, px.stw);
+    float2 *xf = line_fft<false>(fr, o2, px, 1, t, tpr);
     if (valid)
       for (int i = t; i < n; i += tpr) {
         a.dst[base + i] = x[i];
@@ -154,32 +157,9 @@ __device__ __forceinline__ void row_pass_body(const LinePlan &px, const PassArgs
   }
 }
 
-template <int MODE, int NC>
-__global__ void __launch_bounds__(256) row_pass_kernel(LinePlan px, PassArgs a, int tpr, int rpb, long long nrows) {
-  row_pass_body<MODE, NC>(px, a, tpr, rpb, nrows);
-}
-
-// 1000-point rows (the mixed batches' largest non-power-of-two length) run
-// as one row of 200 threads per block with at most 32 registers, so that nine
-// blocks share an SM and a 1000-row pattern takes one wave (the difference
-// map's iteration keeps the general kernel).  Measured on one B200, HIO
-// 1000x1000 per slot: 43.2 us with the general budget (42 registers), 43.6
-// with 40, 39.9 with 32 (a few bytes of spills, more blocks in flight).
-template <int MODE>
-__global__ void __maxnreg__(32)
-    row_pass_kernel_1000(LinePlan px, PassArgs a, int tpr, int rpb, long long nrows) {
-  row_pass_body<MODE, 1000>(px, a, tpr, rpb, nrows);
-}
-
 // ------------------------------------------------------------- column pass
-// byte offset of the stage table behind a column block's buffers (16-byte aligned)
-__host__ __device__ constexpr size_t col_tw_offset(int n, int ct, bool proj) {
-  return ((size_t)2 * n * ct * 8 + (proj ? (size_t)n * ct * 5 : 0) + 15) / 16 * 16;
-}
-
-// compile-time plans read their stage table from shared memory
-template <int MODE, int NC>
-__device__ __forceinline__ void col_pass_body(const LinePlan &pl, const PassArgs &a, int ct, int tpc) {
+template <int MODE>
+__global__ void __launch_bounds__(1024) col_pass_kernel(LinePlan pl, PassArgs a, int ct, int tpc) {
   extern __shared__ float2 smem[];
   const int n = pl.n;
   const int cc = threadIdx.x % ct, t = threadIdx.x / ct;
@@ -195,9 +175,6 @@ __device__ __forceinline__ void col_pass_body(const LinePlan &pl, const PassArgs
   float *AMc = reinterpret_cast<float *>(smem + (size_t)2 * n * ct) + cc;
   uint8_t *FLc = reinterpret_cast<uint8_t *>(reinterpret_cast<float *>(smem + (size_t)2 * n * ct) + (size_t)n * ct) + cc;
   const long long ai0 = PROJ ? lbase % a.n_start : 0;
-  float2 *TW = reinterpret_cast<float2 *>(reinterpret_cast<unsigned char *>(smem) + col_tw_offset(n, ct, PROJ));
-  if constexpr (NC > 0)
-    for (int i = threadIdx.x; i < NC - 1; i += blockDim.x) TW[i] = pl.stw[i];
 
   for (int i = t; i < n; i += tpc) {
     float2 v = make_float2(0.0f, 0.0f);
@@ -219,11 +196,11 @@ __device__ __forceinline__ void col_pass_body(const LinePlan &pl, const PassArgs
 
   float2 *r;
   if constexpr (MODE == COL_FWD) {
-    r = line_fft_sel<false, NC>(A, B, pl, ct, t, tpc, TW);
+    r = line_fft<false>(A, B, pl, ct, t, tpc);
   } else if constexpr (MODE == COL_INV || MODE == COL_INV_SQUARE_F32) {
-    r = line_fft_sel<true, NC>(A, B, pl, ct, t, tpc, TW);
+    r = line_fft<true>(A, B, pl, ct, t, tpc);
   } else {
-    float2 *f = line_fft_sel<false, NC>(A, B, pl, ct, t, tpc, TW);
+    float2 *f = line_fft<false>(A, B, pl, ct, t, tpc);
     if (valid) {
       for (int i = t; i < n; i += tpc) {
         const long long idx = lbase + i * a.estride;
@@ -236,23 +213,10 @@ __device__ __forceinline__ void col_pass_body(const LinePlan &pl, const PassArgs
     }
     __syncthreads();
     float2 *o2 = (f == A) ? B : A;
-    r = line_fft_sel<true, NC>(f, o2, pl, ct, t, tpc, TW);
+    r = line_fft<true>(f, o2, pl, ct, t, tpc);
   }
   if (valid)
     for (int i = t; i < n; i += tpc) a.dst[lbase + i * a.estride] = r[(size_t)i * ct];
-}
-
-template <int MODE, int NC>
-__global__ void __launch_bounds__(1024) col_pass_kernel(LinePlan pl, PassArgs a, int ct, int tpc) {
-  col_pass_body<MODE, NC>(pl, a, ct, tpc);
-}
-
-// 1000-point columns run as four columns of 200 threads per block with at
-// most 32 registers, so that two blocks share an SM (a 1000-column pattern:
-// 250 blocks, one wave)
-template <int MODE>
-__global__ void __maxnreg__(32) col_pass_kernel_1000(LinePlan pl, PassArgs a, int ct, int tpc) {
-  col_pass_body<MODE, 1000>(pl, a, ct, tpc);
 }
 
 // ---------------------------------------------------------------- launchers
@@ -271,60 +235,24 @@ static cudaError_t smem_attr(K k, size_t smem, size_t &done) {
   return e;
 }
 
-// lengths with a compile-time plan in the general kernels (the non-power-of-two
-// sizes of the mixed batches); others use the run-time plan
-#define SPB_CT_LENGTHS(X) X(192) X(384) X(1000)
-// the difference map's row passes also take compile-time plans at powers of
-// two: grids of a few short rows per SM run here rather than in the register
-// kernel (spb_fast.cu), and so does the f1 transform (ROW_DM_F1_FWD)
-#define SPB_CT_LENGTHS_DM(X) X(64) X(128) X(256) X(512) X(1024) X(2048)
-
-template <int MODE, int NC>
-static cudaError_t row_launch_n(const LinePlan &px, const PassArgs &a, cudaStream_t st) {
+template <int MODE>
+static cudaError_t row_launch(const LinePlan &px, const PassArgs &a, cudaStream_t st) {
   const int n = px.n;
-  // compile-time plans: one butterfly per thread, at least two warps per row
-  int tpr = NC > 0 ? (ct_max_butterflies(NC) > 64 ? ct_max_butterflies(NC) : 64) : pow2_at_least((n + 15) / 16);
+  int tpr = pow2_at_least((n + 15) / 16);
   if (tpr > 256) tpr = 256;
-  if (tpr < 1) tpr = 1;
   const long long nrows = a.n / n;
-  int rpb = 256 / tpr;
-  if (NC > 0) {  // no fewer blocks than two per SM when the rows allow it
-    const long long cap = nrows / 296;
-    if (cap < rpb) rpb = cap > 0 ? (int)cap : 1;
-  }
+  const int rpb = 256 / tpr;
   const int nbuf = (MODE == ROW_DM_ITER) ? 4 : 2;
   constexpr bool UPD = (MODE == ROW_ITER || MODE == ROW_DM_ITER);
   // transform buffers, then (UPD) a slab of g0 and rpb*n bytes of flags
   const size_t smem = (size_t)(nbuf + (UPD ? 1 : 0)) * rpb * n * sizeof(float2) + (UPD ? (size_t)rpb * n : 0);
-  auto k = row_pass_kernel<MODE, NC>;
-  if constexpr (NC == 1000 && MODE != ROW_DM_ITER) k = row_pass_kernel_1000<MODE>;
+  auto k = row_pass_kernel<MODE>;
   static size_t done = 0;
   cudaError_t e = smem_attr(k, smem, done);
   if (e != cudaSuccess) return e;
   const long long grid = (nrows + rpb - 1) / rpb;
   k<<<(unsigned)grid, rpb * tpr, smem, st>>>(px, a, tpr, rpb, nrows);
   return cudaGetLastError();
-}
-
-template <int MODE>
-static cudaError_t row_launch(const LinePlan &px, const PassArgs &a, cudaStream_t st) {
-  if (px.stw) {
-    switch (px.n) {
-#define SPB_CASE(n) \
-  case n: return row_launch_n<MODE, n>(px, a, st);
-      SPB_CT_LENGTHS(SPB_CASE)
-#undef SPB_CASE
-    }
-    if constexpr (MODE == ROW_DM_ITER || MODE == ROW_DM_F1_FWD) {
-      switch (px.n) {
-#define SPB_CASE(n) \
-  case n: return row_launch_n<MODE, n>(px, a, st);
-        SPB_CT_LENGTHS_DM(SPB_CASE)
-#undef SPB_CASE
-      }
-    }
-  }
-  return row_launch_n<MODE, 0>(px, a, st);
 }
 
 // The 8-point kernels for a pass of `nlines` lines of length n: asked for
@@ -349,6 +277,8 @@ cudaError_t launch_row(int mode, const LinePlan &px, const PassArgs &a, cudaStre
   }
   const cudaError_t fe = launch_row_fast(mode, px, a, st);
   if (fe != cudaErrorNotSupported) return fe;
+  const cudaError_t me = launch_row_mixed(mode, px, a, st);
+  if (me != cudaErrorNotSupported) return me;
   switch (mode) {
     case ROW_FWD: return row_launch<ROW_FWD>(px, a, st);
     case ROW_FWD_DEPHASE: return row_launch<ROW_FWD_DEPHASE>(px, a, st);
@@ -364,66 +294,32 @@ cudaError_t launch_row(int mode, const LinePlan &px, const PassArgs &a, cudaStre
   return cudaErrorInvalidValue;
 }
 
-// Columns per block SPB_TUNE_COL_WIDTH may ask of the general projection pass
-// for the compile-time-plan lengths: a power of two up to 16 that keeps one
-// butterfly per thread within 1024 threads.
+// Columns per block SPB_TUNE_COL_WIDTH may ask of the projection pass of the
+// mixed-radix lines of 192, 384 and 1000 points (the knob's documented lengths).
 bool general_col_width_ok(int n, int w) {
   if (w < 1 || w > 16 || (w & (w - 1))) return false;
-  switch (n) {
-#define SPB_CASE(len) \
-  case len: return w * ct_max_butterflies(len) <= 1024;
-    SPB_CT_LENGTHS(SPB_CASE)
-#undef SPB_CASE
-  }
-  return false;
+  return (n == 192 && w <= 16) || (n == 384 && w <= 8) || (n == 1000 && w <= 4);
 }
 
-template <int MODE, int NC>
-static cudaError_t col_launch_n(const LinePlan &pl, const PassArgs &a, cudaStream_t st) {
+template <int MODE>
+static cudaError_t col_launch(const LinePlan &pl, const PassArgs &a, cudaStream_t st) {
   const int n = pl.n;
   constexpr bool PROJ = (MODE == COL_PROJECT || MODE == COL_PROJECT_NOFC);
   int ct = 4096 / (n > 0 ? n : 1);
   if (ct > 16) ct = 16;
   if (ct < 1) ct = 1;
-  int tpc = NC > 0 ? ct_max_butterflies(NC) : pow2_at_least((n + 15) / 16);
-  if (NC > 0 && tpc * ct > 1024) ct = 1024 / tpc > 0 ? 1024 / tpc : 1;  // keep one butterfly per thread
-  // projection with a compile-time plan: four columns per block (a full
-  // 32-byte sector per row, and more blocks than the wider default gives a
-  // single pattern).  Measured on one B200, HIO per slot at 16/8/4/2/1 columns:
-  // 192^2 13.6/12.2/11.6/11.9/12.6 us, 384^2 -/16.4/14.9/15.9/17.8 us, 1000^2
-  // (four by default) 39.2, 49.2 at 2, 57.7 at 1.  A launch-shape knob may
-  // ask for another number of columns per block.
-  if (NC > 0 && PROJ) {
-    if (ct > 4) ct = 4;
-    if (a.col_width > 0 && general_col_width_ok(NC, a.col_width)) ct = a.col_width;
-  }
+  int tpc = pow2_at_least((n + 15) / 16);
   if (tpc * ct > 1024) tpc = 1024 / ct;
   if (tpc * ct < 32) tpc = 32 / ct;
-  // two transform buffers, then (projection) n*ct amplitudes and n*ct flag
-  // bytes, then (compile-time plans) the n - 1 entries of the stage table
-  const size_t smem = NC > 0 ? col_tw_offset(n, ct, PROJ) + (size_t)(NC - 1) * sizeof(float2)
-                             : (size_t)2 * n * ct * sizeof(float2) + (PROJ ? (size_t)n * ct * (sizeof(float) + 1) : 0);
-  auto k = col_pass_kernel<MODE, NC>;
-  if constexpr (NC == 1000) k = col_pass_kernel_1000<MODE>;
+  // two transform buffers, then (projection) n*ct amplitudes and n*ct flag bytes
+  const size_t smem = (size_t)2 * n * ct * sizeof(float2) + (PROJ ? (size_t)n * ct * (sizeof(float) + 1) : 0);
+  auto k = col_pass_kernel<MODE>;
   static size_t done = 0;
   cudaError_t e = smem_attr(k, smem, done);
   if (e != cudaSuccess) return e;
   dim3 grid((a.ncols + ct - 1) / ct, a.nouter);
   k<<<grid, ct * tpc, smem, st>>>(pl, a, ct, tpc);
   return cudaGetLastError();
-}
-
-template <int MODE>
-static cudaError_t col_launch(const LinePlan &pl, const PassArgs &a, cudaStream_t st) {
-  if (pl.stw) {
-    switch (pl.n) {
-#define SPB_CASE(n) \
-  case n: return col_launch_n<MODE, n>(pl, a, st);
-      SPB_CT_LENGTHS(SPB_CASE)
-#undef SPB_CASE
-    }
-  }
-  return col_launch_n<MODE, 0>(pl, a, st);
 }
 
 cudaError_t launch_col(int mode, const LinePlan &pl, int line_len, const PassArgs &a, cudaStream_t st) {
@@ -435,6 +331,8 @@ cudaError_t launch_col(int mode, const LinePlan &pl, int line_len, const PassArg
   (void)line_len;
   const cudaError_t fe = launch_col_fast(mode, pl, a, st);
   if (fe != cudaErrorNotSupported) return fe;
+  const cudaError_t me = launch_col_mixed(mode, pl, a, st);
+  if (me != cudaErrorNotSupported) return me;
   switch (mode) {
     case COL_FWD: return col_launch<COL_FWD>(pl, a, st);
     case COL_INV: return col_launch<COL_INV>(pl, a, st);

@@ -31,6 +31,63 @@ __device__ __forceinline__ float2 apply_constraints(float2 g, uint8_t f, int c) 
   return g;
 }
 
+// The HIO, RAAR or ER update (src/phasing.c:1111-1219) and the real-space
+// constraints (src/phasing.c:1026-1059) of one pixel without a branch: outside
+// the support out = gp * a + g0 * b with (a, b) = (-beta, 1) for HIO (g0 * 1 is
+// g0, and g0 - x is -x + g0), (1 - 2 beta, beta) for RAAR, 0 for ER; inside,
+// the constraints as a lower limit (0 or -inf) of each part.
+struct UpdateRule {
+  float a, b;
+  float lim_x, lim_y;  // a part below its limit becomes 0, or its absolute value (flip)
+  bool er, flip, real;
+  float2 z;            // (-0, -0), see spb_mixed.cuh
+};
+__device__ __forceinline__ UpdateRule update_rule(const PassArgs &p, float beta, float neg0) {
+  UpdateRule r;
+  r.er = p.alg == ALG_ER;
+  r.a = p.alg == ALG_HIO ? -beta : fsub(1.0f, fmul(2.0f, beta));  // 1 - 2*beta in float, as the reference
+  r.b = p.alg == ALG_HIO ? 1.0f : beta;
+  const int c = p.constraints;
+  const float none = -INFINITY;
+  r.real = (c & (C_REAL | C_POS_REAL)) != 0;
+  r.lim_x = !(c & C_REAL) && (c & (C_POS_REAL | C_POS_COMPLEX)) ? 0.0f : none;
+  r.lim_y = !r.real && (c & C_POS_COMPLEX) ? 0.0f : none;
+  r.flip = (c & C_FLIP) != 0;
+  r.z = make_float2(neg0, neg0);
+  return r;
+}
+__device__ __forceinline__ float2 update_point(float2 gp, float2 g0, bool inside, const UpdateRule &r) {
+  const float2 x = __ffma2_rn(gp, make_float2(r.a, r.a), r.z), y = __ffma2_rn(g0, make_float2(r.b, r.b), r.z);
+  float2 o = __fadd2_rn(x, y);
+  if (r.er) o = make_float2(0.0f, 0.0f);
+  float2 i = gp;
+  if (i.x < r.lim_x) i.x = r.flip ? -i.x : 0.0f;
+  if (i.y < r.lim_y) i.y = r.flip ? -i.y : 0.0f;
+  if (r.real) i.y = 0.0f;
+  return inside ? i : o;
+}
+// scale_cmul_dev in packed arithmetic
+__device__ __forceinline__ float2 scale_point(float2 v, float s, float2 z) {
+  const float2 p = __ffma2_rn(v, make_float2(s, s), z);
+  const float2 q = __ffma2_rn(make_float2(v.y, v.x), make_float2(0.0f, 0.0f), z);
+  return __ffma2_rn(q, make_float2(-1.0f, 1.0f), p);
+}
+
+// The difference map's update (src/phasing.c:1222-1274): rho and fv the
+// unnormalised backward transforms of Y and Yf.  x / size as the reference
+// divides; a multiply by the exact reciprocal when the size is a power of two.
+__device__ __forceinline__ float2 dm_point(float2 rho, float2 fv, float2 g0, uint8_t f, float beta, const PassArgs &a) {
+  auto div_size = [&](float x) { return a.inv_size_pow2 != 0.0f ? fmul(x, a.inv_size_pow2) : __fdiv_rn(x, a.size_f); };
+  float2 g = g0;
+  if (f & FLAG_INSIDE) {
+    g.x = fadd(g0.x, fmul(beta, fsub(div_size(fmul(a.one_p_g2, rho.x)), fmul(a.gamma2, g0.x))));
+    g.y = fadd(g0.y, fmul(beta, fsub(div_size(fmul(a.one_p_g2, rho.y)), fmul(a.gamma2, g0.y))));
+  }
+  g.x = fsub(g.x, div_size(fmul(beta, fv.x)));
+  g.y = fsub(g.y, div_size(fmul(beta, fv.y)));
+  return apply_constraints(g, f, a.constraints);
+}
+
 // ---------------------------------------------------------------------------
 // Branch-free correctly rounded square root, reciprocal and quotient of floats
 // (the bits of __fsqrt_rn, __frcp_rn and __fdiv_rn), from Newton-Raphson steps
@@ -117,6 +174,49 @@ __device__ __forceinline__ float2 project_vals(float2 G, uint8_t f, float amp, l
   return G;
 }
 
+// project_vals of U pixels: without a branch per pixel when every amplitude
+// (amp_ok) and every measured |G|^2 lie in the domains of the branch-free
+// roundings, where the quotient is always finite; else pixel by pixel.
+template <int U, bool FC>
+__device__ __forceinline__ void project_many(float2 (&G)[U], const uint8_t (&f)[U], const float (&amp)[U],
+                                             const long long (&ai)[U], bool amp_ok, const PassArgs &a) {
+  float s2[U];
+  bool fast = amp_ok;
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    if (FC && (a.constraints & C_CENTROSYM)) G[u].y = 0.0f;
+    s2[u] = fadd(fmul(G[u].y, G[u].y), fmul(G[u].x, G[u].x));
+    fast = fast && (!(f[u] & FLAG_MEASURED) || sqrt_rn_nb_domain(s2[u]));
+  }
+  if (fast) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const float m = div_rn_nb(amp[u], sqrt_rn_nb(s2[u]));
+      if (f[u] & FLAG_MEASURED) G[u] = make_float2(fmul(G[u].x, m), fmul(G[u].y, m));
+    }
+  } else {
+#pragma unroll 1
+    for (int u = 0; u < U; u++) {
+      float2 g = G[0];
+      uint8_t fu = f[0];
+      float au = amp[0];
+      long long iu = ai[0];
+#pragma unroll
+      for (int v = 1; v < U; v++)
+        if (u == v) {
+          g = G[v];
+          fu = f[v];
+          au = amp[v];
+          iu = ai[v];
+        }
+      g = project_vals(g, fu, au, iu, a, false);
+#pragma unroll
+      for (int v = 0; v < U; v++)
+        if (u == v) G[v] = g;
+    }
+  }
+}
+
 // the same at pixel idx, operands read from global memory
 __device__ __forceinline__ float2 project(float2 G, long long idx, const PassArgs &a, bool fourier_constraints) {
   const long long ai = idx % a.n_start;  // amplitude-side arrays hold one start
@@ -136,15 +236,19 @@ __device__ __forceinline__ float gauss_factor(float dx, float dy, float dz, cons
   return __double2float_rn(__ddiv_rn(exp(arg), (double)a.n_f));
 }
 
-__device__ __forceinline__ float2 gauss_mult(float2 F, long long gidx, const PassArgs &a) {
-  const long long idx = gidx % a.n_start;  // position within its start
-  const long long nxy = (long long)a.nx * a.ny;
-  const int z = (int)(idx / nxy), y = (int)((idx % nxy) / a.nx), x = (int)(idx % a.nx);
+// F times the factor of pixel (x, y, z)
+__device__ __forceinline__ float2 blur_point(float2 F, int x, int y, int z, const PassArgs &a) {
   const int dx = min(a.nx - x, x), dy = min(a.ny - y, y), dz = min(a.nz - z, z);
   // the factor table of this blur (gauss_table_kernel) holds the same floats
   const float m = a.blur_tab ? a.blur_tab[((long long)dz * (a.ny / 2 + 1) + dy) * (a.nx / 2 + 1) + dx]
                              : gauss_factor((float)dx, (float)dy, (float)dz, a);
   return scale_cmul_dev(F, m);
+}
+
+__device__ __forceinline__ float2 gauss_mult(float2 F, long long gidx, const PassArgs &a) {
+  const long long idx = gidx % a.n_start;  // position within its start
+  const long long nxy = (long long)a.nx * a.ny;
+  return blur_point(F, (int)(idx % a.nx), (int)((idx % nxy) / a.nx), (int)(idx / nxy), a);
 }
 
 }  // namespace spb
