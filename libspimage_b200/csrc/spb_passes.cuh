@@ -87,6 +87,15 @@ __host__ __device__ constexpr int bits_stride() {
   return C == 1 ? proj_words(N) : proj_words(N) + ((((C <= 8 ? 32 / C : 4) - proj_words(N) % 32) + 32) % 32);
 }
 
+// multiprocessors of the device
+inline cudaError_t device_sms(int *n) {
+  static int nsm = 0;
+  cudaError_t e = cudaSuccess;
+  if (!nsm) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, 0);
+  *n = nsm;
+  return e;
+}
+
 // dynamic shared memory limit of kernel K raised to at least smem (once per size)
 template <auto K>
 static cudaError_t ensure_smem(size_t smem) {
