@@ -20,6 +20,39 @@ namespace spb {
 // column x) of X sits at i*P + x; a row's exchanges use the padded positions
 // of its own P slots, a column's exchanges use its own elements (stride P).
 namespace reg {
+// The twiddles of a stage on a thread's points in packed products; k = 0 takes
+// none.  They run under a branch (a select costs two instructions a point in
+// packed form), where T is a multiple of NS one for the J butterflies of a
+// thread, which then share k and the table's loads, elsewhere only for a
+// butterfly whose T j is a multiple of NS.
+template <int N, int R, int NS, bool INV>
+__device__ __forceinline__ void twiddle_points(float2 (&v)[16], int t, const float2 *stw) {
+  constexpr int T = N / 16, J = 16 / R;
+  if constexpr (NS > 1 && T % NS == 0) {
+    const int k = t & (NS - 1);
+    if (k) {
+#pragma unroll
+      for (int m = 1; m < R; m++) {
+        const float2 w = stw[(m - 1) * NS + k];  // shared-memory stage table
+#pragma unroll
+        for (int j = 0; j < J; j++) v[j + m * J] = packed::cmulw(v[j + m * J], w.x, INV ? -w.y : w.y);
+      }
+    }
+  } else if constexpr (NS > 1) {
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const int k = (t + T * j) & (NS - 1);
+      if ((T * j) % NS != 0 || k) {
+#pragma unroll
+        for (int m = 1; m < R; m++) {
+          const float2 w = stw[(m - 1) * NS + k];
+          v[j + m * J] = packed::cmulw(v[j + m * J], w.x, INV ? -w.y : w.y);
+        }
+      }
+    }
+  }
+}
+
 template <int N, int S, int NS, bool INV, int STRIDE>
 struct PStages {
   // storage address of line index i: padded within a row (STRIDE 0) or down a column
@@ -29,6 +62,7 @@ struct PStages {
     constexpr int T = N / 16;
     constexpr int J = 16 / R;
     constexpr bool LAST = (S == plan_len(N) - 1);
+    twiddle_points<N, R, NS, INV>(v, t, stw);
 #pragma unroll
     for (int j = 0; j < J; j++) {
       float2 a[R];
@@ -36,16 +70,10 @@ struct PStages {
       for (int m = 0; m < R; m++) a[m] = v[j + m * J];
       const int b = t + T * j;
       const int k = b & (NS - 1);
-      if constexpr (NS > 1) {
-#pragma unroll
-        for (int m = 1; m < R; m++) {
-          float2 w = stw[(m - 1) * NS + k];
-          if (INV) w.y = -w.y;
-          const float2 p = cmulw(a[m], w.x, w.y);
-          a[m] = k ? p : a[m];
-        }
-      }
-      bfly<R, INV>(a);
+      if constexpr (R == 16) packed::bf16<INV>(a);
+      else if constexpr (R == 8) packed::bf8<INV>(a);
+      else if constexpr (R == 4) packed::bf4<INV>(a[0], a[1], a[2], a[3]);
+      else bfly<R, INV>(a);
       if constexpr (LAST) {
 #pragma unroll
         for (int m = 0; m < R; m++) v[j + m * J] = a[m];
@@ -95,7 +123,7 @@ __global__ void __launch_bounds__(N * N / 16, persist_min_blocks<N>())
     const float2 *g0 = (cur ? gbuf0 : gbuf1) + off;  // the previous model
     float2 *g1 = (cur ? gbuf1 : gbuf0) + off;        // the new one
     const float beta = a.alg == ALG_ER ? 0.0f : (a.beta_tab ? a.beta_tab[*a.beta_base + it] : a.beta);
-    const float one_m2b = fsub(1.0f, fmul(2.0f, beta));
+    const UpdateRule rule = update_rule(a, beta);
     {  // column pass: column c, thread t of its T
       const int c = threadIdx.x % N, t = threadIdx.x / N;
       float2 v[16];
@@ -118,26 +146,9 @@ __global__ void __launch_bounds__(N * N / 16, persist_min_blocks<N>())
       __syncthreads();  // every row read before its slots serve as exchange space
       reg::PStages<N, 0, 1, true, 0>::run(v, Xs + r * P, t, tw_s);
       const bool last = keep_gp && it == iters - 1;
-#pragma unroll
-      for (int q = 0; q < 16; q++) {
-        const int idx = r * N + t + T * q;
-        const float2 gpv = scale_cmul_dev(v[q], a.inv_n);
-        if (last) a.gp[off + idx] = gpv;
-        const uint8_t f = flags[idx];
-        float2 g = make_float2(0.0f, 0.0f);
-        if (f & FLAG_INSIDE) {
-          g = gpv;
-        } else if (a.alg == ALG_HIO) {
-          const float2 o = g0[idx];
-          g = make_float2(fsub(o.x, fmul(gpv.x, beta)), fsub(o.y, fmul(gpv.y, beta)));
-        } else if (a.alg == ALG_RAAR) {
-          const float2 o = g0[idx];
-          g = make_float2(fadd(fmul(gpv.x, one_m2b), fmul(o.x, beta)), fadd(fmul(gpv.y, one_m2b), fmul(o.y, beta)));
-        }
-        g = apply_constraints(g, f, a.constraints);
-        g1[idx] = g;
-        v[q] = g;
-      }
+      const int idx = r * N + t;
+      update_points(v, g0 + idx, flags + idx, last ? a.gp + off + idx : nullptr, g1 + idx, rule, a,
+                    [](int q) { return T * q; });
       reg::PStages<N, 0, 1, false, 0>::run(v, Xs + r * P, t, tw_s);
 #pragma unroll
       for (int q = 0; q < 16; q++) Xs[r * P + t + T * q] = v[q];

@@ -169,6 +169,118 @@ __device__ __forceinline__ void bf5(float2 *a) {
   }
 }
 
+// ------------------------------------------------------- packed arithmetic
+// The products and the radix-4, 8 and 16 butterflies in packed f32x2
+// instructions (sm_100).  Each lane rounds exactly as the scalar intrinsic and
+// the halves of an operand may be swapped, repeated or negated (both) for
+// free: a twiddle product is three instructions (six above), t + i d one.  A
+// packed product is fma(a, b, -0): an exact product plus -0 rounds once, to the
+// product's own bits (signed zeros included).  A packed multiply would not do:
+// it is contracted with the packed add that follows (measured: one-ulp
+// differences in 31 % of twiddle products; none in 2^28 with this form).  The
+// -0 sits in constant memory so that the compiler cannot fold it away.  The
+// packed forms take 10-30 registers more (pairs for the constants), so kernels
+// that live on their occupancy keep the forms above: used in packed form, the
+// row pass of 64 starts of 512^2 went from 111 to 118 us.
+namespace packed {
+static __constant__ float2 kNeg0 = {-0.0f, -0.0f};
+__device__ __forceinline__ float2 cswap(float2 a) { return make_float2(a.y, a.x); }
+// both parts times their factor
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __ffma2_rn(a, b, kNeg0); }
+__device__ __forceinline__ float2 mul2(float2 a, float b) { return __ffma2_rn(a, make_float2(b, b), kNeg0); }
+// (a.re*w.re - a.im*w.im, a.re*w.im + a.im*w.re), each product rounded
+__device__ __forceinline__ float2 cmulw(float2 a, float wr, float wi) {
+  return __ffma2_rn(mul2(cswap(a), wi), make_float2(-1.0f, 1.0f), mul2(a, wr));
+}
+// im*im + re*re
+__device__ __forceinline__ float cabs2(float2 a) {
+  const float2 p = mul2(a, a);
+  return fadd(p.y, p.x);
+}
+// t + W4 d and t - W4 d (W4 = -i forward, +i backward): fma(d, +-1, t) rounds
+// like the add or subtract it stands for
+template <bool INV>
+__device__ __forceinline__ float2 add_w4(float2 t, float2 d) {
+  return __ffma2_rn(cswap(d), INV ? make_float2(-1.0f, 1.0f) : make_float2(1.0f, -1.0f), t);
+}
+template <bool INV>
+__device__ __forceinline__ float2 sub_w4(float2 t, float2 d) {
+  return __ffma2_rn(cswap(d), INV ? make_float2(1.0f, -1.0f) : make_float2(-1.0f, 1.0f), t);
+}
+template <bool INV>
+__device__ __forceinline__ float2 mul_w4(float2 a) {
+  return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+}
+// W8 a and W8^3 a: (re + im, im - re) C8 forward, (re - im, im + re) C8
+// backward, and the same swapped and signed
+template <bool INV>
+__device__ __forceinline__ float2 mul_w8_1(float2 a) {
+  return mul2(add_w4<INV>(a, a), SPB_C8);
+}
+template <bool INV>
+__device__ __forceinline__ float2 mul_w8_3(float2 a) {
+  return mul2(cswap(add_w4<INV>(a, a)), INV ? make_float2(-SPB_C8, SPB_C8) : make_float2(SPB_C8, -SPB_C8));
+}
+
+
+template <bool INV>
+__device__ __forceinline__ void bf4(float2 &a0, float2 &a1, float2 &a2, float2 &a3) {
+  const float2 t0 = cadd(a0, a2), t1 = csub(a0, a2), t2 = cadd(a1, a3), d = csub(a1, a3);
+  a0 = cadd(t0, t2);
+  a1 = add_w4<INV>(t1, d);
+  a2 = csub(t0, t2);
+  a3 = sub_w4<INV>(t1, d);
+}
+// bf4 with a2 still to be multiplied by W4
+template <bool INV>
+__device__ __forceinline__ void bf4_w4(float2 &a0, float2 &a1, float2 &a2, float2 &a3) {
+  const float2 t0 = add_w4<INV>(a0, a2), t1 = sub_w4<INV>(a0, a2), t2 = cadd(a1, a3), d = csub(a1, a3);
+  a0 = cadd(t0, t2);
+  a1 = add_w4<INV>(t1, d);
+  a2 = csub(t0, t2);
+  a3 = sub_w4<INV>(t1, d);
+}
+
+template <bool INV>
+__device__ __forceinline__ void bf8(float2 *a) {
+  bf4<INV>(a[0], a[2], a[4], a[6]);
+  bf4<INV>(a[1], a[3], a[5], a[7]);
+  const float2 o1 = mul_w8_1<INV>(a[3]), o3 = mul_w8_3<INV>(a[7]);
+  const float2 t[8] = {cadd(a[0], a[1]), cadd(a[2], o1), add_w4<INV>(a[4], a[5]), cadd(a[6], o3),
+                       csub(a[0], a[1]), csub(a[2], o1), sub_w4<INV>(a[4], a[5]), csub(a[6], o3)};
+#pragma unroll
+  for (int k = 0; k < 8; k++) a[k] = t[k];
+}
+
+template <bool INV>
+__device__ __forceinline__ void bf16(float2 *a) {
+  const float s = INV ? -1.0f : 1.0f;
+#pragma unroll
+  for (int q2 = 0; q2 < 4; q2++) bf4<INV>(a[q2], a[q2 + 4], a[q2 + 8], a[q2 + 12]);
+  a[1 + 4 * 1] = cmulw(a[1 + 4 * 1], SPB_C16, -SPB_S16 * s);
+  a[1 + 4 * 2] = mul_w8_1<INV>(a[1 + 4 * 2]);
+  a[1 + 4 * 3] = cmulw(a[1 + 4 * 3], SPB_S16, -SPB_C16 * s);
+  a[2 + 4 * 1] = mul_w8_1<INV>(a[2 + 4 * 1]);
+  a[2 + 4 * 3] = mul_w8_3<INV>(a[2 + 4 * 3]);
+  a[3 + 4 * 1] = cmulw(a[3 + 4 * 1], SPB_S16, -SPB_C16 * s);
+  a[3 + 4 * 2] = mul_w8_3<INV>(a[3 + 4 * 2]);
+  a[3 + 4 * 3] = cmulw(a[3 + 4 * 3], -SPB_C16, SPB_S16 * s);
+#pragma unroll
+  for (int k1 = 0; k1 < 4; k1++) {
+    if (k1 == 2) bf4_w4<INV>(a[4 * k1], a[4 * k1 + 1], a[4 * k1 + 2], a[4 * k1 + 3]);  // a[10] times W4
+    else bf4<INV>(a[4 * k1], a[4 * k1 + 1], a[4 * k1 + 2], a[4 * k1 + 3]);
+  }
+  float2 t[16];
+#pragma unroll
+  for (int k1 = 0; k1 < 4; k1++)
+#pragma unroll
+    for (int k2 = 0; k2 < 4; k2++) t[k1 + 4 * k2] = a[4 * k1 + k2];
+#pragma unroll
+  for (int k = 0; k < 16; k++) a[k] = t[k];
+}
+
+}  // namespace packed
+
 template <int R, bool INV>
 __device__ __forceinline__ void bfly(float2 *a) {
   if constexpr (R == 2) bf2<INV>(a[0], a[1]);

@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(512, 2)
           at(rb + 8 * i) = y;
         }
       } else if (valid) {
-        const UpdateRule rule = update_rule(a, beta, mp.neg0);
+        const UpdateRule rule = update_rule(a, beta);
         for (int i0 = L.t; i0 < n; i0 += 4 * tpl) {
           uint8_t f[4];
           float2 g[4];
@@ -90,16 +90,16 @@ __global__ void __launch_bounds__(512, 2)
             g[u] = zero;
             if (i < n) {
               f[u] = fl[i];
-              if (!rule.er) g[u] = g0[i];
+              if (a.alg != ALG_ER) g[u] = g0[i];
             }
           }
 #pragma unroll
           for (int u = 0; u < 4; u++) {
             const int i = i0 + u * tpl, m = r + L.base + 8 * i;
             if (i < n) {
-              const float2 w = scale_point(at(m), a.inv_n, rule.z);
+              const float2 w = packed::cmulw(at(m), a.inv_n, 0.0f);
               if (gp) gp[i] = w;
-              const float2 x = update_point(w, g[u], f[u] & FLAG_INSIDE, rule);
+              const float2 x = rule.rare ? update_point_any(w, g[u], f[u], rule, a) : update_point(w, g[u], f[u], rule);
               g1[i] = x;
               at(m) = x;
             }

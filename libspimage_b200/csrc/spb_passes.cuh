@@ -76,6 +76,28 @@ __device__ __forceinline__ float2 project_with(float2 G, float amp, bool measure
   return make_float2(amp, 0.0f);
 }
 
+// The update of a thread's U points after the inverse transform: v becomes the
+// new model, gp (when set) and g1 take the model before projection and the
+// new model.  Point q lies off(q) behind g0, fl, gp and g1.
+template <int U, class Off>
+__device__ __forceinline__ void update_points(float2 (&v)[U], const float2 *g0, const uint8_t *fl, float2 *gp, float2 *g1,
+                                              const UpdateRule &r, const PassArgs &a, Off off) {
+#pragma unroll
+  for (int q = 0; q < U; q++) v[q] = packed::cmulw(v[q], a.inv_n, 0.0f);  // scale_cmul_dev
+  if (gp)
+#pragma unroll
+    for (int q = 0; q < U; q++) gp[off(q)] = v[q];
+  if (r.rare) {
+#pragma unroll
+    for (int q = 0; q < U; q++) v[q] = update_point_any(v[q], g0[off(q)], fl[off(q)], r, a);
+  } else {
+#pragma unroll
+    for (int q = 0; q < U; q++) v[q] = update_point(v[q], g0[off(q)], fl[off(q)], r);
+  }
+#pragma unroll
+  for (int q = 0; q < U; q++) g1[off(q)] = v[q];
+}
+
 // words per line of the measured-bit bitmap (a multiple of 4 words)
 __host__ __device__ constexpr int proj_words(int n) { return ((n + 127) / 128) * 4; }
 template <int N, int C>

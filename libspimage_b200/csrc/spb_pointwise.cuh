@@ -32,19 +32,19 @@ __device__ __forceinline__ float2 apply_constraints(float2 g, uint8_t f, int c) 
 }
 
 // The HIO, RAAR or ER update (src/phasing.c:1111-1219) and the real-space
-// constraints (src/phasing.c:1026-1059) of one pixel without a branch: outside
-// the support out = gp * a + g0 * b with (a, b) = (-beta, 1) for HIO (g0 * 1 is
-// g0, and g0 - x is -x + g0), (1 - 2 beta, beta) for RAAR, 0 for ER; inside,
-// the constraints as a lower limit (0 or -inf) of each part.
+// constraints (src/phasing.c:1026-1059) of one pixel.  Outside the support out
+// = gp * a + g0 * b with (a, b) = (-beta, 1) for HIO (g0 * 1 is g0, and g0 - x is
+// -x + g0), (1 - 2 beta, beta) for RAAR, 0 for ER; inside, the constraints as a
+// lower limit (0 or -inf) of each part.  ER and flipping positivity take a
+// branch that is uniform over the grid; the rest has none.
 struct UpdateRule {
   float a, b;
-  float lim_x, lim_y;  // a part below its limit becomes 0, or its absolute value (flip)
-  bool er, flip, real;
-  float2 z;            // (-0, -0), see spb_mixed.cuh
+  float lim_x, lim_y;  // a part below its limit becomes 0
+  bool real;           // the imaginary part becomes 0
+  bool rare;           // ER or flipping positivity
 };
-__device__ __forceinline__ UpdateRule update_rule(const PassArgs &p, float beta, float neg0) {
+__device__ __forceinline__ UpdateRule update_rule(const PassArgs &p, float beta) {
   UpdateRule r;
-  r.er = p.alg == ALG_ER;
   r.a = p.alg == ALG_HIO ? -beta : fsub(1.0f, fmul(2.0f, beta));  // 1 - 2*beta in float, as the reference
   r.b = p.alg == ALG_HIO ? 1.0f : beta;
   const int c = p.constraints;
@@ -52,25 +52,23 @@ __device__ __forceinline__ UpdateRule update_rule(const PassArgs &p, float beta,
   r.real = (c & (C_REAL | C_POS_REAL)) != 0;
   r.lim_x = !(c & C_REAL) && (c & (C_POS_REAL | C_POS_COMPLEX)) ? 0.0f : none;
   r.lim_y = !r.real && (c & C_POS_COMPLEX) ? 0.0f : none;
-  r.flip = (c & C_FLIP) != 0;
-  r.z = make_float2(neg0, neg0);
+  r.rare = p.alg == ALG_ER || (c & C_FLIP);
   return r;
 }
-__device__ __forceinline__ float2 update_point(float2 gp, float2 g0, bool inside, const UpdateRule &r) {
-  const float2 x = __ffma2_rn(gp, make_float2(r.a, r.a), r.z), y = __ffma2_rn(g0, make_float2(r.b, r.b), r.z);
-  float2 o = __fadd2_rn(x, y);
-  if (r.er) o = make_float2(0.0f, 0.0f);
-  float2 i = gp;
-  if (i.x < r.lim_x) i.x = r.flip ? -i.x : 0.0f;
-  if (i.y < r.lim_y) i.y = r.flip ? -i.y : 0.0f;
-  if (r.real) i.y = 0.0f;
-  return inside ? i : o;
+// r.rare false
+__device__ __forceinline__ float2 update_point(float2 gp, float2 g0, uint8_t f, const UpdateRule &r) {
+  const float2 o = cadd(packed::mul2(gp, r.a), packed::mul2(g0, r.b));
+  const float x = gp.x < r.lim_x ? 0.0f : gp.x;
+  const float y = (gp.y < r.lim_y) | r.real ? 0.0f : gp.y;
+  const bool inside = f & FLAG_INSIDE;
+  return make_float2(inside ? x : o.x, inside ? y : o.y);
 }
-// scale_cmul_dev in packed arithmetic
-__device__ __forceinline__ float2 scale_point(float2 v, float s, float2 z) {
-  const float2 p = __ffma2_rn(v, make_float2(s, s), z);
-  const float2 q = __ffma2_rn(make_float2(v.y, v.x), make_float2(0.0f, 0.0f), z);
-  return __ffma2_rn(q, make_float2(-1.0f, 1.0f), p);
+// any rule
+__device__ __forceinline__ float2 update_point_any(float2 gp, float2 g0, uint8_t f, const UpdateRule &r,
+                                                   const PassArgs &p) {
+  float2 g = gp;
+  if (!(f & FLAG_INSIDE)) g = p.alg == ALG_ER ? make_float2(0.0f, 0.0f) : cadd(packed::mul2(gp, r.a), packed::mul2(g0, r.b));
+  return apply_constraints(g, f, p.constraints);
 }
 
 // The difference map's update (src/phasing.c:1222-1274): rho and fv the
@@ -138,6 +136,24 @@ __device__ __forceinline__ float rcp_rn_nb(float b) {
   const float y0 = rcp_seed(b);
   return __fmaf_rn(__fmaf_rn(-b, y0, 1.0f), y0, y0);
 }
+// sqrt_rn_nb and then div_rn_nb of two values at once, the steps in packed
+// arithmetic (each half rounds as the scalar step)
+__device__ __forceinline__ float2 div_sqrt_rn_nb2(float2 a, float2 x) {
+  const float2 t = make_float2(rsqrt_seed(x.x), rsqrt_seed(x.y));
+  float2 g = packed::mul2(x, t);
+  float2 h = packed::mul2(t, 0.5f);
+  const float2 r = __ffma2_rn(make_float2(-g.x, -g.y), h, make_float2(0.5f, 0.5f));
+  g = __ffma2_rn(g, r, g);
+  h = __ffma2_rn(h, r, h);
+  const float2 d = __ffma2_rn(make_float2(-g.x, -g.y), g, x);
+  const float2 b = __ffma2_rn(d, h, g);  // the square roots
+  const float2 nb = make_float2(-b.x, -b.y);
+  const float2 y0 = make_float2(rcp_seed(b.x), rcp_seed(b.y));
+  const float2 y = __ffma2_rn(__ffma2_rn(nb, y0, make_float2(1.0f, 1.0f)), y0, y0);
+  const float2 q0 = packed::mul2(a, y);
+  const float2 q1 = __ffma2_rn(__ffma2_rn(nb, q0, a), y, q0);
+  return __ffma2_rn(__ffma2_rn(nb, q1, a), y, q1);
+}
 // a / b for b in [2^-63, 2^63] and a in div_rn_nb_domain
 __device__ __forceinline__ float div_rn_nb(float a, float b) {
   const float y = rcp_rn_nb(b);
@@ -185,14 +201,15 @@ __device__ __forceinline__ void project_many(float2 (&G)[U], const uint8_t (&f)[
 #pragma unroll
   for (int u = 0; u < U; u++) {
     if (FC && (a.constraints & C_CENTROSYM)) G[u].y = 0.0f;
-    s2[u] = fadd(fmul(G[u].y, G[u].y), fmul(G[u].x, G[u].x));
+    s2[u] = packed::cabs2(G[u]);
     fast = fast && (!(f[u] & FLAG_MEASURED) || sqrt_rn_nb_domain(s2[u]));
   }
   if (fast) {
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const float m = div_rn_nb(amp[u], sqrt_rn_nb(s2[u]));
-      if (f[u] & FLAG_MEASURED) G[u] = make_float2(fmul(G[u].x, m), fmul(G[u].y, m));
+    for (int u = 0; u < U; u += 2) {
+      const float2 m = div_sqrt_rn_nb2(make_float2(amp[u], amp[u + 1]), make_float2(s2[u], s2[u + 1]));
+      if (f[u] & FLAG_MEASURED) G[u] = packed::mul2(G[u], m.x);
+      if (f[u + 1] & FLAG_MEASURED) G[u + 1] = packed::mul2(G[u + 1], m.y);
     }
   } else {
 #pragma unroll 1

@@ -42,6 +42,13 @@
 
 namespace spb {
 namespace split {
+using packed::add_w4;
+using packed::cswap;
+using packed::mul2;
+using packed::mul_w4;
+using packed::mul_w8_1;
+using packed::mul_w8_3;
+
 
 __host__ __device__ constexpr int plan_radix(int n, int s) {
   int r[16] = {0};
@@ -76,18 +83,12 @@ __device__ __forceinline__ float2 shfl16(float2 v) {
   return make_float2(__shfl_xor_sync(0xffffffffu, v.x, 16), __shfl_xor_sync(0xffffffffu, v.y, 16));
 }
 
-// W8^1 (h = 0) or W8^3 (h = 1) from shared products: the roundings of
-// mul_w8_1 / mul_w8_3 exactly (negation is exact)
+// W8^1 (h = 0) or W8^3 (h = 1): mul_w8_1 or mul_w8_3 from the shared sums
 template <bool INV>
 __device__ __forceinline__ float2 mul_w8_13(float2 a, bool h) {
-  const float p = fmul(fadd(a.x, a.y), SPB_C8);
-  if (!INV) {
-    const float q = fmul(fsub(a.y, a.x), SPB_C8);
-    return h ? make_float2(q, -p) : make_float2(p, q);
-  } else {
-    const float q = fmul(fsub(a.x, a.y), SPB_C8);
-    return h ? make_float2(-p, q) : make_float2(q, p);
-  }
+  const float2 v = add_w4<INV>(a, a);
+  const float c = INV ? -SPB_C8 : SPB_C8;
+  return mul2(sel(h, cswap(v), v), sel(h, make_float2(c, -c), make_float2(SPB_C8, SPB_C8)));
 }
 
 // Radix-16 butterfly split over the pair (see the file comment); in and out
@@ -96,13 +97,13 @@ template <bool INV>
 __device__ __forceinline__ void bf16_half(float2 (&a)[8], bool h) {
   const float s = INV ? -1.0f : 1.0f;
   // first layer: DFT4 over q1 for q2 = 2h + e (registers e + 2*q1)
-  bf4<INV>(a[0], a[2], a[4], a[6]);
-  bf4<INV>(a[1], a[3], a[5], a[7]);
+  packed::bf4<INV>(a[0], a[2], a[4], a[6]);
+  packed::bf4<INV>(a[1], a[3], a[5], a[7]);
   // internal twiddles W16^(q2*k1) of the rows q2 = 2h + e, register e + 2*k1
   // e = 1: q2 = 1 (W^1, W^2, W^3) or q2 = 3 (W^3, W^6, W^9)
-  a[3] = cmulw(a[3], h ? SPB_S16 : SPB_C16, h ? -SPB_C16 * s : -SPB_S16 * s);
+  a[3] = packed::cmulw(a[3], h ? SPB_S16 : SPB_C16, h ? -SPB_C16 * s : -SPB_S16 * s);
   a[5] = mul_w8_13<INV>(a[5], h);
-  a[7] = cmulw(a[7], h ? -SPB_C16 : SPB_S16, h ? SPB_S16 * s : -SPB_C16 * s);
+  a[7] = packed::cmulw(a[7], h ? -SPB_C16 : SPB_S16, h ? SPB_S16 * s : -SPB_C16 * s);
   // e = 0: q2 = 0 (identity) or q2 = 2 (W^2, W^4, W^6)
   a[2] = sel(h, mul_w8_1<INV>(a[2]), a[2]);
   a[4] = sel(h, mul_w4<INV>(a[4]), a[4]);
@@ -122,7 +123,7 @@ __device__ __forceinline__ void bf16_half(float2 (&a)[8], bool h) {
       in[e] = sel(h, r, lo);
       in[2 + e] = sel(h, hi, r);
     }
-    bf4<INV>(in[0], in[1], in[2], in[3]);
+    packed::bf4<INV>(in[0], in[1], in[2], in[3]);
     // X[k1 + 4*k2] with k1 = 2h + f: register f + 2*k2
 #pragma unroll
     for (int k2 = 0; k2 < 4; k2++) a[f + 2 * k2] = in[k2];
@@ -137,8 +138,8 @@ __device__ __forceinline__ void bf8_half(const float2 (&a_in)[8], float2 (&o)[8]
 #pragma unroll
   for (int i = 0; i < 8; i++) a[i] = a_in[i];
   // DFT4 over the even (h = 0) or odd (h = 1) inputs of both butterflies
-  bf4<INV>(a[0], a[2], a[4], a[6]);
-  bf4<INV>(a[1], a[3], a[5], a[7]);
+  packed::bf4<INV>(a[0], a[2], a[4], a[6]);
+  packed::bf4<INV>(a[1], a[3], a[5], a[7]);
   // odd outputs o_1, o_2, o_3 times W8^1, W4^1, W8^3 (h = 1 only)
 #pragma unroll
   for (int e = 0; e < 2; e++) {
@@ -170,19 +171,13 @@ struct Stages {
       const int b = t;
       const int k = b & (NS - 1);
       if constexpr (NS > 1) {
+        if (k) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const int m = 2 * hh + mi0(i);
-          if (i == 0) {  // m = 0 (h = 0) takes no twiddle
-            float2 w = stw[(m > 0 ? m - 1 : 0) * NS + k];
-            if (INV) w.y = -w.y;
-            const float2 p = cmulw(v[i], w.x, w.y);
-            v[i] = (k && m) ? p : v[i];
-          } else {
-            float2 w = stw[(m - 1) * NS + k];
-            if (INV) w.y = -w.y;
-            const float2 p = cmulw(v[i], w.x, w.y);
-            v[i] = k ? p : v[i];
+          for (int i = 0; i < 8; i++) {
+            const int m = 2 * hh + mi0(i);
+            const float2 w = stw[(m > 0 ? m - 1 : 0) * NS + k];
+            const float2 p = packed::cmulw(v[i], w.x, INV ? -w.y : w.y);
+            v[i] = i > 0 ? p : sel(h, p, v[i]);  // m = 0 (i = 0, h = 0) takes no twiddle
           }
         }
       }
@@ -204,14 +199,17 @@ struct Stages {
       static_assert(NS % 16 == 0, "a radix-8 stage follows a radix-16 stage here");
       // register e + 2k: butterfly j = e (b = t + T*e), input m = h + 2k
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        const int e = i & 1, m = hh + 2 * (i >> 1);
-        const int b = t + T * e;
-        const int k = b & (NS - 1);
-        float2 w = stw[(m > 0 ? m - 1 : 0) * NS + k];
-        if (INV) w.y = -w.y;
-        const float2 p = cmulw(v[i], w.x, w.y);
-        v[i] = (k && m) ? p : v[i];
+      for (int e = 0; e < 2; e++) {
+        const int k = (t + T * e) & (NS - 1);
+        if (k) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const int m = hh + 2 * j;
+            const float2 w = stw[(m > 0 ? m - 1 : 0) * NS + k];
+            const float2 p = packed::cmulw(v[e + 2 * j], w.x, INV ? -w.y : w.y);
+            v[e + 2 * j] = j > 0 ? p : sel(h, p, v[e]);  // m = 0 (j = 0, h = 0) takes no twiddle
+          }
+        }
       }
       float2 o[8];
       bf8_half<INV>(v, o, h);
@@ -227,15 +225,15 @@ struct Stages {
         const int b = t + T * (2 * hh + e);
         const int k = b & (NS - 1);
         if constexpr (NS > 1) {
+          if (k) {
 #pragma unroll
-          for (int m = 1; m < 4; m++) {
-            float2 w = stw[(m - 1) * NS + k];
-            if (INV) w.y = -w.y;
-            const float2 p = cmulw(v[e + 2 * m], w.x, w.y);
-            v[e + 2 * m] = k ? p : v[e + 2 * m];
+            for (int m = 1; m < 4; m++) {
+              const float2 w = stw[(m - 1) * NS + k];
+              v[e + 2 * m] = packed::cmulw(v[e + 2 * m], w.x, INV ? -w.y : w.y);
+            }
           }
         }
-        bf4<INV>(v[e], v[e + 2], v[e + 4], v[e + 6]);
+        packed::bf4<INV>(v[e], v[e + 2], v[e + 4], v[e + 6]);
         if constexpr (!LAST) {
           const int base = (b / NS) * NS * 4 + k;
 #pragma unroll
@@ -281,16 +279,17 @@ __device__ __forceinline__ void project8(float2 (&v)[8], const float *amp_l, con
     const int i = t + T * (2 * hh + split::mi0(q));
     const unsigned meas = (meas_l[i >> 5] >> (i & 31)) & 1u;
     mm |= meas << q;
-    s2[q] = fadd(fmul(v[q].y, v[q].y), fmul(v[q].x, v[q].x));
+    s2[q] = packed::cabs2(v[q]);
     fast = fast && (!meas || sqrt_rn_nb_domain(s2[q]));
   }
   if (fast) {
 #pragma unroll
-    for (int q = 0; q < 8; q++) {
-      const float amp = amp_l[t + T * (2 * hh + split::mi0(q))];
-      const float m = div_rn_nb(amp, sqrt_rn_nb(s2[q]));
-      const float2 p = isfinite(m) ? make_float2(fmul(v[q].x, m), fmul(v[q].y, m)) : make_float2(amp, 0.0f);
-      if ((mm >> q) & 1u) v[q] = p;
+    for (int q = 0; q < 8; q += 2) {
+      // inside the domains the quotient of a measured point is finite
+      const float2 amp = make_float2(amp_l[t + T * (2 * hh + split::mi0(q))], amp_l[t + T * (2 * hh + split::mi0(q + 1))]);
+      const float2 m = div_sqrt_rn_nb2(amp, make_float2(s2[q], s2[q + 1]));
+      if ((mm >> q) & 1u) v[q] = packed::mul2(v[q], m.x);
+      if ((mm >> (q + 1)) & 1u) v[q + 1] = packed::mul2(v[q + 1], m.y);
     }
   } else {
 #pragma unroll
@@ -306,7 +305,7 @@ __device__ __forceinline__ void project8(float2 (&v)[8], const float *amp_l, con
 // kernel: [twiddles N][LPB exchange lines][LPB rows of g0 unless G0LATE]
 // [LPB rows of flags].
 template <int N, bool G0LATE>
-__global__ void __launch_bounds__(512) row_split_kernel(PassArgs a, const float2 *__restrict__ stw, int nrows) {
+__global__ void __launch_bounds__(512, 2) row_split_kernel(PassArgs a, const float2 *__restrict__ stw, int nrows) {
   constexpr int T = N / 16;
   constexpr int TL = 2 * T;  // threads per line
   constexpr int S = N + N / 16;
@@ -343,8 +342,7 @@ __global__ void __launch_bounds__(512) row_split_kernel(PassArgs a, const float2
   for (int i = 0; i < 8; i++) v[i] = valid ? a.src[base + T * split::mi0(i)] : make_float2(0.0f, 0.0f);
   cp_async_wait_all();
   __syncthreads();
-  const float beta = iter_beta(a);
-  const float one_m2b = fsub(1.0f, fmul(2.0f, beta));  // 1 - 2*beta in float, as the reference
+  const UpdateRule rule = update_rule(a, iter_beta(a));
   split::fft<N, true>(v, line, t, h, tw_s);
   if constexpr (G0LATE) {
     // g0 of the block's rows into their exchange lines: the transform's last
@@ -367,29 +365,8 @@ __global__ void __launch_bounds__(512) row_split_kernel(PassArgs a, const float2
   const int lo = t + 2 * hh * T;  // line index of register 0
   const float2 *g0r = G0LATE ? line + lo : g0_s + lr * N + lo;
   const uint8_t *flr = fl_s + lr * N + lo;
-  float2 *gp = a.gp;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const int off = T * split::mi0(i);
-    float2 g = make_float2(0.0f, 0.0f);
-    if (valid) {
-      const float2 gpv = scale_cmul_dev(v[i], a.inv_n);
-      if (gp) gp[base + off] = gpv;
-      const uint8_t f = flr[off];
-      if (f & FLAG_INSIDE) {
-        g = gpv;
-      } else if (a.alg == ALG_HIO) {
-        const float2 g0 = g0r[off];
-        g = make_float2(fsub(g0.x, fmul(gpv.x, beta)), fsub(g0.y, fmul(gpv.y, beta)));
-      } else if (a.alg == ALG_RAAR) {
-        const float2 g0 = g0r[off];
-        g = make_float2(fadd(fmul(gpv.x, one_m2b), fmul(g0.x, beta)), fadd(fmul(gpv.y, one_m2b), fmul(g0.y, beta)));
-      }
-      g = apply_constraints(g, f, a.constraints);
-      a.g1[base + off] = g;
-    }
-    v[i] = g;
-  }
+  if (valid)
+    update_points(v, g0r, flr, a.gp ? a.gp + base : nullptr, a.g1 + base, rule, a, [](int i) { return T * split::mi0(i); });
   if constexpr (G0LATE) __syncthreads();  // every g0 read done before the forward transform writes the lines
   split::fft<N, false>(v, line, t, h, tw_s);
   pdl_release();
@@ -402,7 +379,7 @@ __global__ void __launch_bounds__(512) row_split_kernel(PassArgs a, const float2
 // Block: C columns x 2T threads; lane l = c + C*tl + 16*h (C divides 16), so a
 // warp loads C adjacent columns of 16/C rows for each half; t = tl + (16/C)*w.
 template <int N, int MODE, int C>
-__global__ void __launch_bounds__(512) col_split_kernel(PassArgs a, const float2 *__restrict__ stw) {
+__global__ void __launch_bounds__(512, 2) col_split_kernel(PassArgs a, const float2 *__restrict__ stw) {
   constexpr int T = N / 16;
   constexpr int S = N + N / 16 + (C > 1 ? 16 / C : 0);
   constexpr int TPW = 16 / C;  // t values per warp half
