@@ -1237,6 +1237,25 @@ static bool persist_auto(const spb_ctx *c) {
   return c->nx <= 64 && c->nb >= nsm;
 }
 
+// The difference map's two projections of a 2-D pattern, X to Y and Xf to Yf,
+// in one launch where that pays (launch_col).  Returns 1 when it ran, 0 when
+// the two run one after the other, -1 on error.
+static int project_pair(spb_ctx *c, PassArgs a) {
+  if (c->nz != 1 || c->ny <= 1 || c->nb > kMaxGridY) return 0;
+  const LinePlan *pl = nullptr;
+  col_geometry(c, 1, a, &pl);
+  a.src = c->X;
+  a.dst = c->Y;
+  a.src2 = c->Xf;
+  a.dst2 = c->Yf;
+  if (prof_begin(c)) return -1;
+  const cudaError_t e = launch_col(COL_PROJECT_PAIR, *pl, pl->n, a, c->st);
+  if (e == cudaErrorNotSupported) return 0;
+  CK(e);
+  c->launches++;
+  return prof_end(c, 10 + COL_PROJECT) ? -1 : 1;
+}
+
 // One iteration of every start: g0 <- g1 (buffer roles swap), X -> Y
 // (projection pass) -> row pass writing g1 and the next X.  `a` carries the
 // algorithm scalars.
@@ -1245,9 +1264,11 @@ static int one_iteration(spb_ctx *c, PassArgs a, float2 *gp_out) {
   a.g0 = c->g[c->cur ^ 1];
   a.g1 = c->g[c->cur];
   a.gp = gp_out;
-  if (middle(c, COL_PROJECT, c->X, c->Y, a)) return -1;
+  const int pair = a.alg == ALG_DM ? project_pair(c, a) : 0;
+  if (pair < 0) return -1;
+  if (!pair && middle(c, COL_PROJECT, c->X, c->Y, a)) return -1;
   if (a.alg == ALG_DM) {
-    if (middle(c, COL_PROJECT_NOFC, c->Xf, c->Yf, a)) return -1;
+    if (!pair && middle(c, COL_PROJECT_NOFC, c->Xf, c->Yf, a)) return -1;
     a.src = c->Y;
     a.src2 = c->Yf;
     a.dst = c->X;

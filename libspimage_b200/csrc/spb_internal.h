@@ -39,6 +39,7 @@ enum ColMode : int {
   COL_PROJECT_NOFC = 3,  // fwd, projection only (difference-map f1), inv
   COL_BLUR = 4,          // fwd, Gaussian multiplier, inv
   COL_INV_SQUARE_F32 = 5,  // inv of (real32^2 + 0i) input (Patterson)
+  COL_PROJECT_PAIR = 6,    // COL_PROJECT of src to dst and COL_PROJECT_NOFC of src2 to dst2 in one launch
 };
 
 struct PassArgs {

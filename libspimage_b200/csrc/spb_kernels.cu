@@ -329,6 +329,16 @@ cudaError_t launch_col(int mode, const LinePlan &pl, int line_len, const PassArg
     if (se != cudaErrorNotSupported) return se;
   }
   (void)line_len;
+  if (mode == COL_PROJECT_PAIR) {
+    // where the launches of one image leave SMs idle: 8-point lines and lines
+    // without a register kernel; the others are as fast one after the other
+    if (want_split(a, pl.n, (long long)a.ncols * a.nouter)) {
+      const cudaError_t se = launch_col_split(mode, pl, a, st);
+      if (se != cudaErrorNotSupported) return se;
+    }
+    if ((pl.n & (pl.n - 1)) == 0) return cudaErrorNotSupported;
+    return launch_col_mixed(mode, pl, a, st);
+  }
   const cudaError_t fe = launch_col_fast(mode, pl, a, st);
   if (fe != cudaErrorNotSupported) return fe;
   const cudaError_t me = launch_col_mixed(mode, pl, a, st);

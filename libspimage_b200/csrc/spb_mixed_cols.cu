@@ -10,7 +10,7 @@ namespace mix {
 template <int MODE>
 __global__ void __launch_bounds__(512, 2)
     col_kernel(const __grid_constant__ MixPlan mp, const __grid_constant__ PassArgs a, int nl, int lg) {
-  constexpr bool PROJ = MODE == COL_PROJECT || MODE == COL_PROJECT_NOFC;
+  constexpr bool PROJ = MODE == COL_PROJECT || MODE == COL_PROJECT_NOFC || MODE == COL_PROJECT_PAIR;
   constexpr bool MID = PROJ || MODE == COL_BLUR;  // forward, pointwise, inverse; else one transform
   constexpr bool FWD = MID || MODE == COL_FWD;
   const int n = mp.n;
@@ -22,9 +22,10 @@ __global__ void __launch_bounds__(512, 2)
   const long long base = o * a.ostride + c0;  // the block's first point
   const int es = (int)a.estride;              // a start has fewer than 2^31 points
   const bool valid = c < a.ncols;
-  const float2 *src = a.src + base;
+  const bool second = MODE == COL_PROJECT_PAIR && blockIdx.z;  // the second image
+  const float2 *src = (second ? a.src2 : a.src) + base;
   const float *f32 = a.f32src + base;
-  float2 *dst = a.dst + base;
+  float2 *dst = (second ? a.dst2 : a.dst) + base;
   stage_tables(mp, tw);
   pdl_wait();
   const float2 zero = make_float2(0.0f, 0.0f);
@@ -67,6 +68,7 @@ __global__ void __launch_bounds__(512, 2)
           for (int u = 0; u < 4; u++) {
             const int i = i0 + u * L.tpl;
             G[u] = i < n ? at(r + L.base + i * L.es) : zero;
+            if (MODE == COL_PROJECT_PAIR && !second && (a.constraints & C_CENTROSYM)) G[u].y = 0.0f;
           }
           project_many<4, MODE == COL_PROJECT>(G, f, amp, ai, amp_ok, a);
 #pragma unroll
@@ -94,10 +96,11 @@ template <int MODE>
 static cudaError_t launch_col(const LinePlan &pl, const PassArgs &a, cudaStream_t st) {
   // four columns a block (a 32-byte sector of every row); eight when that
   // still gives two blocks per SM
-  const long long lines = (long long)a.ncols * a.nouter;
+  constexpr int IMAGES = MODE == COL_PROJECT_PAIR ? 2 : 1;
+  const long long lines = (long long)a.ncols * a.nouter * IMAGES;
   const MixPlan &mp = choose_plan(pl, lines);
   int nl = lines / 8 >= 2 * num_sms() ? 8 : 4;
-  if ((MODE == COL_PROJECT || MODE == COL_PROJECT_NOFC) && a.col_width > 0) nl = a.col_width;
+  if ((MODE == COL_PROJECT || MODE == COL_PROJECT_NOFC || MODE == COL_PROJECT_PAIR) && a.col_width > 0) nl = a.col_width;
   while (nl > 1 && smem_bytes(mp, nl) > kMixSmem) nl >>= 1;
   const size_t smem = smem_bytes(mp, nl);
   if (smem > kMixSmem) return cudaErrorNotSupported;
@@ -107,7 +110,7 @@ static cudaError_t launch_col(const LinePlan &pl, const PassArgs &a, cudaStream_
   if (e != cudaSuccess) return e;
   int threads = (nl * threads_per_line(mp, lines, 512 / nl) + 31) / 32 * 32;
   if (threads > 512) threads = 512;
-  const dim3 grid((a.ncols + nl - 1) / nl, a.nouter);
+  const dim3 grid((a.ncols + nl - 1) / nl, a.nouter, IMAGES);
   return launch_maybe_pdl(col_kernel<MODE>, grid, dim3(threads), smem, st, a.pdl != 0, mp, a, nl, lg);
 }
 
@@ -120,6 +123,7 @@ cudaError_t launch_col_mixed(int mode, const LinePlan &pl, const PassArgs &a, cu
     case COL_INV: return mix::launch_col<COL_INV>(pl, a, st);
     case COL_PROJECT: return mix::launch_col<COL_PROJECT>(pl, a, st);
     case COL_PROJECT_NOFC: return mix::launch_col<COL_PROJECT_NOFC>(pl, a, st);
+    case COL_PROJECT_PAIR: return mix::launch_col<COL_PROJECT_PAIR>(pl, a, st);
     case COL_BLUR: return mix::launch_col<COL_BLUR>(pl, a, st);
     case COL_INV_SQUARE_F32: return mix::launch_col<COL_INV_SQUARE_F32>(pl, a, st);
   }

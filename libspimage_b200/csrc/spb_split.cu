@@ -376,6 +376,7 @@ __global__ void __launch_bounds__(512, 2) row_split_kernel(PassArgs a, const flo
 }
 
 // --------------------------------------------------------- column kernel
+// COL_PROJECT_PAIR: blocks of grid.z = 1 take the second image.
 // Block: C columns x 2T threads; lane l = c + C*tl + 16*h (C divides 16), so a
 // warp loads C adjacent columns of 16/C rows for each half; t = tl + (16/C)*w.
 template <int N, int MODE, int C>
@@ -392,6 +393,9 @@ __global__ void __launch_bounds__(512, 2) col_split_kernel(PassArgs a, const flo
   const int col0 = blockIdx.x * C;
   const int col = col0 + c;
   const bool valid = col < a.ncols;
+  const bool second = MODE == COL_PROJECT_PAIR && blockIdx.z;
+  const float2 *src = second ? a.src2 : a.src;
+  float2 *dst = second ? a.dst2 : a.dst;
   float2 *tw_s = sm;
   float2 *line = sm + N + c * S;
   constexpr int W = proj_words(N);
@@ -418,16 +422,19 @@ __global__ void __launch_bounds__(512, 2) col_split_kernel(PassArgs a, const flo
   pdl_wait();
   float2 v[8];
 #pragma unroll
-  for (int i = 0; i < 8; i++) v[i] = valid ? a.src[lbase + split::mi0(i) * qstride] : make_float2(0.0f, 0.0f);
+  for (int i = 0; i < 8; i++) v[i] = valid ? src[lbase + split::mi0(i) * qstride] : make_float2(0.0f, 0.0f);
   cp_async_wait_all();
   __syncthreads();
   split::fft<N, false>(v, line, t, h, tw_s);
+  if (MODE == COL_PROJECT_PAIR && !second && (a.constraints & C_CENTROSYM))
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i].y = 0.0f;
   if (valid) project8<T, MODE == COL_PROJECT>(v, amp_s + c * SA, meas_s + c * SW, t, hh, lbase, qstride, a);
   split::fft<N, true>(v, line, t, h, tw_s);
   pdl_release();
   if (valid)
 #pragma unroll
-    for (int i = 0; i < 8; i++) a.dst[lbase + split::mi0(i) * qstride] = v[i];
+    for (int i = 0; i < 8; i++) dst[lbase + split::mi0(i) * qstride] = v[i];
 }
 
 // ---------------------------------------------------------------- launch
@@ -464,7 +471,7 @@ static cudaError_t col_split_launch(const LinePlan &pl, const PassArgs &a, cudaS
                       (size_t)C * amp_stride<N, C>() * sizeof(float) + (size_t)C * bits_stride<N, C>() * sizeof(uint32_t);
   cudaError_t e = ensure_smem<col_split_kernel<N, MODE, C>>(smem);
   if (e != cudaSuccess) return e;
-  dim3 grid((a.ncols + C - 1) / C, a.nouter);
+  dim3 grid((a.ncols + C - 1) / C, a.nouter, MODE == COL_PROJECT_PAIR ? 2 : 1);
   return launch_maybe_pdl(col_split_kernel<N, MODE, C>, grid, dim3(C * TL), smem, st, a.pdl != 0, a, pl.stw);
 }
 
@@ -482,6 +489,10 @@ cudaError_t launch_row_split(int mode, const LinePlan &px, const PassArgs &a, cu
 }
 
 cudaError_t launch_col_split(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st) {
+  if (pl.stw && mode == COL_PROJECT_PAIR) {  // the lengths the built-in choice runs here
+    if (pl.n == 256) return col_split_launch<256, COL_PROJECT_PAIR>(pl, a, st);
+    if (pl.n == 512) return col_split_launch<512, COL_PROJECT_PAIR>(pl, a, st);
+  }
   if (!pl.stw || (mode != COL_PROJECT && mode != COL_PROJECT_NOFC)) return cudaErrorNotSupported;
   const bool fc = mode == COL_PROJECT;
   switch (pl.n) {
