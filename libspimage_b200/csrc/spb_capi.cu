@@ -127,9 +127,9 @@ int make_axis(Axis &ax, int n) {
       if (!s.kind)
         for (int e = 0; e < s.r; e++) st.push_back(h[(size_t)e * (n / s.r)]);
     }
-  CK(cudaMalloc(&ax.tw, sizeof(float2) * ((size_t)n + st.size())));
-  CK(cudaMemcpy(ax.tw, h.data(), sizeof(float2) * (size_t)n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(ax.tw + n, st.data(), sizeof(float2) * st.size(), cudaMemcpyHostToDevice));
+  h.insert(h.end(), st.begin(), st.end());
+  CK(cudaMalloc(&ax.tw, sizeof(float2) * h.size()));
+  CK(cudaMemcpy(ax.tw, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
   ax.lp.tw = ax.tw;
   ax.lp.stw = ax.tw + n;
   for (MixPlan &mp : ax.mix) {
@@ -253,6 +253,10 @@ struct spb_ctx {
   int x_valid = 0, xf_valid = 0;
   float xf_gamma1 = 0.0f;
   int tune[SPB_TUNE_KNOBS] = {};  // launch-shape choices (0: built-in)
+  // one-shot contexts (transform_ctx): the one allocation that every buffer
+  // lies in, its size and how much of it is given out; null otherwise
+  unsigned char *slab = nullptr;
+  size_t slab_bytes = 0, slab_used = 0;
 };
 
 namespace {
@@ -586,6 +590,46 @@ extern "C" int spb_ctx_create_batch(spb_ctx **out, int nx, int ny, int nz, int n
   return 0;
 }
 
+// A context for one-shot calls on host buffers (spb_fft_host, spb_blur_host,
+// spb_prtf_host): a stream, the transforms' tables and one allocation of `bytes`
+// that carve() shares out, instead of the phasing state's 17 allocations, its
+// pinned rings and 130 events, which took longer than the transforms
+// themselves (an FFT of 900x1200: 10.3 ms a call, 0.1 of it on the GPU).
+const size_t kCarveAlign = 256;
+static size_t carved(size_t bytes) { return (bytes + kCarveAlign - 1) / kCarveAlign * kCarveAlign; }
+static void *carve(spb_ctx *c, size_t bytes) {
+  void *p = c->slab + c->slab_used;
+  c->slab_used += carved(bytes);
+  return c->slab_used <= c->slab_bytes ? p : nullptr;
+}
+static int transform_ctx(spb_ctx **out, int nx, int ny, int nz, size_t bytes) {
+  *out = nullptr;
+  if (check_dims(nx, ny, nz, 1)) return -1;
+  spb_ctx *c = new spb_ctx();
+  c->nx = nx;
+  c->ny = ny;
+  c->nz = nz;
+  c->n = c->ntot = (long long)nx * ny * nz;
+  c->slab_bytes = bytes + carved(sizeof(int));
+  int rc = 0;
+  cudaError_t e = cudaStreamCreateWithFlags(&c->own_st, cudaStreamNonBlocking);
+  if (e != cudaSuccess) rc = fail("cudaStreamCreate: %s", cudaGetErrorString(e));
+  c->st = c->own_st;
+  if (!rc && (e = cudaMalloc(&c->slab, c->slab_bytes)) != cudaSuccess)
+    rc = fail("cudaMalloc(%zu): %s", c->slab_bytes, cudaGetErrorString(e));
+  if (!rc) {
+    c->err_flag = (int *)carve(c, sizeof(int));
+    if (cudaMemsetAsync(c->err_flag, 0, sizeof(int), c->st) != cudaSuccess) rc = fail("cudaMemsetAsync");
+  }
+  if (!rc && (make_axis(c->ax, nx) || make_axis(c->ay, ny) || make_axis(c->az, nz))) rc = -1;
+  if (rc) {
+    spb_ctx_destroy(c);
+    return rc;
+  }
+  *out = c;
+  return 0;
+}
+
 extern "C" int spb_ctx_create(spb_ctx **out, int nx, int ny, int nz) {
   return spb_ctx_create_batch(out, nx, ny, nz, 1);
 }
@@ -650,6 +694,13 @@ extern "C" long long spb_ctx_footprint(int nx, int ny, int nz, int nb, int dm) {
 extern "C" void spb_ctx_destroy(spb_ctx *c) {
   if (!c) return;
   if (c->st) cudaStreamSynchronize(c->st);
+  if (c->slab) {  // a one-shot context: every buffer lies in the slab
+    for (void *p : {(void *)c->slab, (void *)c->ax.tw, (void *)c->ay.tw, (void *)c->az.tw})
+      if (p) cudaFree(p);
+    cudaStreamDestroy(c->own_st);
+    delete c;
+    return;
+  }
   void *ptrs[] = {c->amp, c->amin, c->amax, c->pamp, c->flags, c->g[0], c->g[1], c->X, c->Y, c->Xf, c->Yf,
                   c->gp, c->T, c->absb, c->gtab, c->sel, c->red, c->nonfinite, c->err_flag, c->ax.tw, c->ay.tw,
                   c->az.tw,
@@ -2015,8 +2066,10 @@ extern "C" int spb_ctx_support_count(spb_ctx *c, long long *count) {
 // ------------------------------------------------------------ one-shot API
 extern "C" int spb_fft_host(int nx, int ny, int nz, int sign, const float *in, float *out) {
   spb_ctx *c = nullptr;
-  if (spb_ctx_create(&c, nx, ny, nz)) return -1;
-  const size_t nc = sizeof(float2) * (size_t)c->n;
+  const size_t nc = sizeof(float2) * (size_t)nx * ny * nz;
+  if (transform_ctx(&c, nx, ny, nz, 2 * carved(nc))) return -1;
+  c->T = (float2 *)carve(c, nc);
+  c->Y = (float2 *)carve(c, nc);
   int rc = 0;
   if (upload(c, c->T, in, nc)) rc = -1;
   PassArgs a = base_args(c);
@@ -2037,8 +2090,12 @@ extern "C" int spb_fft_host(int nx, int ny, int nz, int sign, const float *in, f
 
 extern "C" int spb_blur_host(int nx, int ny, int nz, const float *in, float radius, float *out) {
   spb_ctx *c = nullptr;
-  if (spb_ctx_create(&c, nx, ny, nz)) return -1;
-  const size_t nc = sizeof(float2) * (size_t)c->n;
+  if (check_dims(nx, ny, nz, 1)) return -1;
+  const size_t nc = sizeof(float2) * (size_t)nx * ny * nz, ng = sizeof(float) * (size_t)gauss_table_len(nx, ny, nz);
+  if (transform_ctx(&c, nx, ny, nz, 2 * carved(nc) + carved(ng))) return -1;
+  c->T = (float2 *)carve(c, nc);
+  c->Y = (float2 *)carve(c, nc);
+  c->gtab = (float *)carve(c, ng);
   int rc = upload(c, c->Y, in, nc);
   if (!rc) {
     // full complex blur (no dephasing): forward x, middle blur, backward x
@@ -2417,34 +2474,25 @@ int prtf_argmax(spb_ctx *c, const float2 *v, float s, float *bval, long long *bi
 extern "C" int spb_prtf_host(int nx, int ny, int nz, int n, const float *images, const int *supports, int flags,
                              float *prtf, float *super_image, int *super_mask) {
   if (n < 1) return fail("prtf of %d images", n);
+  if (check_dims(nx, ny, nz, 1)) return -1;
   spb_ctx *c = nullptr;
-  if (spb_ctx_create(&c, nx, ny, nz)) return -1;
-  const long long N = c->n;
-  const size_t nc = sizeof(float2) * (size_t)N;
+  const long long N = (long long)nx * ny * nz;
+  const size_t nc = sizeof(float2) * (size_t)N, n4 = sizeof(float) * (size_t)N;
   const int nblk = 296;
-  float2 *scratch = nullptr;
-  int *mask = nullptr, *mask2 = nullptr, *zeros = nullptr, *smask = nullptr;
-  float *counts = nullptr, *bval = nullptr, *dprtf = nullptr;
-  long long *bidx = nullptr;
-  double *part = nullptr;
+  if (transform_ctx(&c, nx, ny, nz, 7 * carved(nc) + 6 * carved(n4) + 3 * carved(2 * sizeof(double) * nblk))) return -1;
   std::vector<float> hval(nblk);
   std::vector<long long> hidx(nblk);
   std::vector<double> hpart(2 * nblk);
   int rc = 0;
-  auto alloc = [&](void **p, size_t bytes) {
-    if (!rc && cudaMalloc(p, bytes) != cudaSuccess) rc = fail("prtf: cudaMalloc(%zu) failed", bytes);
-  };
-  alloc((void **)&scratch, nc);
-  alloc((void **)&mask, sizeof(int) * N);
-  alloc((void **)&mask2, sizeof(int) * N);
-  alloc((void **)&zeros, sizeof(int) * N);
-  alloc((void **)&smask, sizeof(int) * N);
-  alloc((void **)&counts, sizeof(float) * N);
-  alloc((void **)&dprtf, sizeof(float) * N);
-  alloc((void **)&bval, sizeof(float) * nblk);
-  alloc((void **)&bidx, sizeof(long long) * nblk);
-  alloc((void **)&part, sizeof(double) * 2 * nblk);
-  float2 *avg = c->g[0], *img = c->g[1], *A = c->X, *B = c->Y, *C = c->T, *sum = c->gp;
+  float2 *avg = (float2 *)carve(c, nc), *img = (float2 *)carve(c, nc), *A = (float2 *)carve(c, nc),
+         *B = (float2 *)carve(c, nc), *C = (float2 *)carve(c, nc), *sum = (float2 *)carve(c, nc),
+         *scratch = (float2 *)carve(c, nc);
+  c->T = C;  // the inverse transforms' scratch
+  int *mask = (int *)carve(c, n4), *mask2 = (int *)carve(c, n4), *zeros = (int *)carve(c, n4), *smask = (int *)carve(c, n4);
+  float *counts = (float *)carve(c, n4), *dprtf = (float *)carve(c, n4);
+  float *bval = (float *)carve(c, sizeof(float) * nblk);
+  long long *bidx = (long long *)carve(c, sizeof(long long) * nblk);
+  double *part = (double *)carve(c, sizeof(double) * 2 * nblk);
   const float inv_n = (float)(1.0 / (double)N);
   const int translate = flags & 1, enantio = flags & 2;
   // image 0: the running sum and the first unit phasors
@@ -2530,9 +2578,6 @@ extern "C" int spb_prtf_host(int nx, int ny, int nz, int n, const float *images,
   if (!rc && super_mask && cudaMemcpyAsync(super_mask, smask, sizeof(int) * N, cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
     rc = fail("prtf: download");
   if (!rc && cudaStreamSynchronize(c->st) != cudaSuccess) rc = fail("prtf: device error");
-  void *ptrs[] = {scratch, mask, mask2, zeros, smask, counts, dprtf, bval, bidx, part};
-  for (void *p : ptrs)
-    if (p) cudaFree(p);
   spb_ctx_destroy(c);
   return rc;
 }
