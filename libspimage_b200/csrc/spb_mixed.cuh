@@ -34,9 +34,9 @@
 // issue (55-59 % issue active at 192^3 before the pointwise loops were made
 // branch-free).  Per iteration slot, the run-time stage loops these kernels
 // replaced / these kernels: HIO 600^2 38 / 21 us, 768^2 51 / 30, 1200^2 96 / 54,
-// 100^3 85 / 48, 192^3 386 / 186, 384^3 3545 / 1843, 1000^2 39.0 / 36.8 (a
-// compile-time plan before), RAAR 650x670 (2.5.5.13 x 2.5.67) 1818 / 68,
-// 257x263 49000 / 104.  Two lines a thread (shared index arithmetic and
+// 100^3 85 / 48, 192^3 386 / 188, 384^3 3545 / 1910, 1000^2 39.0 / 36.4 (a
+// compile-time plan before), RAAR 650x670 (2.5.5.13 x 2.5.67) 1818 / 57,
+// 257x263 49000 / 80.  Two lines a thread (shared index arithmetic and
 // twiddle loads, 128 registers) was slower everywhere: 1000^2 39.6 against
 // 36.0, 8 x 384^2 57.5 against 44.9.
 #pragma once
@@ -231,10 +231,73 @@ __device__ __forceinline__ void stage(int x, int y, const Lay &L, int tw, const 
   }
 }
 
-// A prime stage R >= 7: y_m = a_0 + sum_q a_q W_R^(mq mod R), added left to
-// right on the twiddled inputs.  A thread computes outputs m and R - m of one
-// butterfly (m = 0: the plain sum); neighbouring threads take neighbouring
-// butterflies, so a warp reads the table at few places.
+// The outputs of a prime stage from its twiddled inputs: y_m = a_0 + sum_q a_q
+// W_R^(mq mod R), added left to right.  A task is output m and output R - m
+// (m = 0: the plain sum) of JB butterflies, b and b + (nb + 1) / 2: the index
+// mq mod R, the table's entry and the loop are shared by them (670-point rows:
+// 1826 -> 1378 instructions a point, 48.8 -> 39.9 us a pass at 650 rows).
+// Neighbouring threads take neighbouring butterflies, so a warp reads the
+// table at few places.
+template <int JB, class Store>
+__device__ __forceinline__ void prime_outputs(int x, int y, const Lay &L, const float2 *__restrict__ wr,
+                                              const MixStep &s, const Dir &g, bool last, Store store) {
+  const int R = s.r, ns = s.ns, nb = s.nb, sin = s.sin * L.es;
+  const int groups = (nb + JB - 1) / JB, half = (R + 1) / 2;
+  for (int t = L.t; t < groups * half; t += L.tpl) {
+    const int m = groups == 1 ? t : (int)__umulhi((unsigned)t, s.group_magic);
+    const int b0 = t - m * groups;
+    int in[JB], out[JB];
+    float2 u[JB], v[JB];
+    bool ok[JB];
+#pragma unroll
+    for (int j = 0; j < JB; j++) {
+      ok[j] = b0 + j * groups < nb;
+      const int b = ok[j] ? b0 + j * groups : b0;
+      const int q0 = ns == 1 ? b : (int)__umulhi((unsigned)b, s.ns_magic);
+      in[j] = x + (b + q0 * s.din) * L.es;
+      out[j] = b + q0 * ns * (R - 1);  // point of output 0
+      u[j] = v[j] = at(in[j]);
+    }
+    if (m == 0) {
+#pragma unroll 4
+      for (int q = 1; q < R; q++)
+#pragma unroll
+        for (int j = 0; j < JB; j++) u[j] = cadd(u[j], at(in[j] += sin));
+    } else {
+      const unsigned step = 8 * m, wrap = 8 * R;
+      unsigned e = 0;  // byte offset of W_R^(mq mod R)
+#pragma unroll 4
+      for (int q = 1; q < R; q++) {
+        e += step;
+        e = min(e, e - wrap);  // unsigned: e - wrap is huge while e < wrap
+        const float2 w = __ldg(reinterpret_cast<const float2 *>(reinterpret_cast<const char *>(wr) + e));
+#pragma unroll
+        for (int j = 0; j < JB; j++) {
+          const float2 aq = at(in[j] += sin);
+          // the products of a term serve both outputs: a w = p + (-i, i) h, a conj(w) = p - (-i, i) h
+          const float2 p = mul(aq, w.x, g), h = mul(swp(aq), w.y, g);
+          u[j] = cadd(u[j], __ffma2_rn(h, neg(g.w), p));
+          v[j] = cadd(v[j], __ffma2_rn(h, g.w, p));
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < JB; j++) {
+      if (!ok[j]) continue;
+      const int ou = out[j] + m * ns, ov = out[j] + (R - m) * ns;
+      if (last) {
+        store(ou, u[j]);
+        if (m) store(ov, v[j]);
+      } else {
+        at(y + ou * L.es) = u[j];
+        if (m) at(y + ov * L.es) = v[j];
+      }
+    }
+  }
+}
+
+// A prime stage R >= 7: its inputs take their twiddles in place, once, then
+// prime_outputs.
 template <class Load, class Store>
 __device__ __forceinline__ void stage_prime(int x, int y, const Lay &L, int tw, const float2 *__restrict__ wr,
                                             const MixStep &s, const Dir &g, bool first, bool last, Load load,
@@ -261,47 +324,17 @@ __device__ __forceinline__ void stage_prime(int x, int y, const Lay &L, int tw, 
     }
     __syncthreads();
   }
-  const int half = (R + 1) / 2;
-  for (int t = L.t; t < nb * half; t += L.tpl) {
-    const int m = nb == 1 ? t : (int)__umulhi((unsigned)t, s.nb_magic);
-    const int b = t - m * nb;
-    const int q0 = ns == 1 ? b : (int)__umulhi((unsigned)b, s.ns_magic);
-    int in = x + (b + q0 * s.din) * L.es;
-    const int out = b + q0 * ns * (R - 1);  // point of output 0
-    const float2 a0 = at(in);
-    float2 u = a0, v = a0;
-    if (m == 0) {
-#pragma unroll 4
-      for (int q = 1; q < R; q++) u = cadd(u, at(in += sin));
-    } else {
-      int e = 0;
-#pragma unroll 4
-      for (int q = 1; q < R; q++) {
-        e += m;
-        e = e >= R ? e - R : e;
-        const float2 w = __ldg(wr + e), aq = at(in += sin);
-        // the products of a term serve both outputs: a w = p + (-i, i) h, a conj(w) = p - (-i, i) h
-        const float2 p = mul(aq, w.x, g), h = mul(swp(aq), w.y, g);
-        u = cadd(u, __ffma2_rn(h, neg(g.w), p));
-        v = cadd(v, __ffma2_rn(h, g.w, p));
-      }
-    }
-    const int ou = out + m * ns, ov = out + (R - m) * ns;
-    if (last) {
-      store(ou, u);
-      if (m) store(ov, v);
-    } else {
-      at(y + ou * L.es) = u;
-      if (m) at(y + ov * L.es) = v;
-    }
-  }
+  if (nb > 1) prime_outputs<2>(x, y, L, wr, s, g, last, store);
+  else prime_outputs<1>(x, y, L, wr, s, g, last, store);
 }
 
 // Every stage of the block's lines, from the buffer at x (or, with from_mem,
 // from load()) to a buffer, or with to_mem to store(); returns the buffer (x
 // or y) of the result.  All threads call it; it synchronises after every step
-// that ends in shared memory.  tw: where the stage tables start.
-template <class Load, class Store>
+// that ends in shared memory.  tw: where the stage tables start.  PRIME: the
+// plan has prime steps (kernels of plans without any leave their code out, for
+// its registers: HIO 600^2 22.3 -> 21.5 us per slot).
+template <bool PRIME, class Load, class Store>
 __device__ __forceinline__ int line_fft(int x, int y, const MixPlan &mp, const Lay &L, int tw, float d, bool from_mem,
                                          bool to_mem, Load load, Store store) {
   const Dir g = make_dir(d, mp.neg0);
@@ -314,7 +347,9 @@ __device__ __forceinline__ int line_fft(int x, int y, const MixPlan &mp, const L
   case mix_kind(r1, r2): stage<r1, r2>(x, y, L, tw, s, g, first, last, load, store); break;
     switch (s.kind) {
       SPB_MIX_KINDS(SPB_MIX_STEP)
-      default: stage_prime(x, y, L, tw, mp.pw + s.pw, s, g, first, last, load, store); break;
+      default:
+        if constexpr (PRIME) stage_prime(x, y, L, tw, mp.pw + s.pw, s, g, first, last, load, store);
+        break;
     }
 #undef SPB_MIX_STEP
     if (!last) __syncthreads();
@@ -343,7 +378,9 @@ inline size_t smem_bytes(const MixPlan &mp, int nl) {
 }
 
 // tasks of a line in a step, and in its widest step
-inline int tasks_of(const MixStep &st) { return st.kind ? st.nb : st.nb * ((st.r + 1) / 2); }
+inline int tasks_of(const MixStep &st) {
+  return st.kind ? st.nb : (st.nb > 1 ? (st.nb + 1) / 2 : 1) * ((st.r + 1) / 2);
+}
 inline int most_tasks(const MixPlan &mp) {
   int t = 1;
   for (int i = 0; i < mp.nsteps; i++) t = tasks_of(mp.step[i]) > t ? tasks_of(mp.step[i]) : t;

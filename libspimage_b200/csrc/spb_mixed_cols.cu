@@ -7,7 +7,7 @@ namespace mix {
 // nl neighbouring columns per block (a power of two, lg its logarithm).
 // Shared memory: two buffers of nl lines of `pitch` points, point i of column p
 // at (i nl + p), then the stage tables.
-template <int MODE>
+template <int MODE, bool PRIME>
 __global__ void __launch_bounds__(512, 2)
     col_kernel(const __grid_constant__ MixPlan mp, const __grid_constant__ PassArgs a, int nl, int lg) {
   constexpr bool PROJ = MODE == COL_PROJECT || MODE == COL_PROJECT_NOFC || MODE == COL_PROJECT_PAIR;
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(512, 2)
 #pragma unroll 1
   for (int ph = FWD ? 0 : 1; ph < 2; ph++) {  // ph 0: forward, 1: inverse
     const bool end = !MID || ph == 1;
-    r = line_fft(r, r ? 0 : by, mp, L, tw, ph ? -1.0f : 1.0f, !MID || ph == 0, end, load, store);
+    r = line_fft<PRIME>(r, r ? 0 : by, mp, L, tw, ph ? -1.0f : 1.0f, !MID || ph == 0, end, load, store);
     if (end) break;
     if constexpr (PROJ) {
       const long long ai0 = base % a.n_start;  // the amplitude side holds one start
@@ -106,12 +106,13 @@ static cudaError_t launch_col(const LinePlan &pl, const PassArgs &a, cudaStream_
   if (smem > kMixSmem) return cudaErrorNotSupported;
   int lg = 0;
   while ((1 << lg) < nl) lg++;
-  const cudaError_t e = ensure_smem<col_kernel<MODE>>(smem);
+  const cudaError_t e = mp.primes ? ensure_smem<col_kernel<MODE, true>>(smem) : ensure_smem<col_kernel<MODE, false>>(smem);
   if (e != cudaSuccess) return e;
   int threads = (nl * threads_per_line(mp, lines, 512 / nl) + 31) / 32 * 32;
   if (threads > 512) threads = 512;
   const dim3 grid((a.ncols + nl - 1) / nl, a.nouter, IMAGES);
-  return launch_maybe_pdl(col_kernel<MODE>, grid, dim3(threads), smem, st, a.pdl != 0, mp, a, nl, lg);
+  return launch_maybe_pdl(mp.primes ? col_kernel<MODE, true> : col_kernel<MODE, false>, grid, dim3(threads), smem, st,
+                          a.pdl != 0, mp, a, nl, lg);
 }
 
 }  // namespace mix

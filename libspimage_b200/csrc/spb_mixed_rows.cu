@@ -9,7 +9,7 @@ namespace mix {
 // nl lines per block, tpl threads each: one row a line, or in the difference
 // map's iteration lines 2j and 2j + 1 the rows of Y and Yf.  Shared memory: two
 // buffers of nl lines of `pitch` points, then the stage tables.
-template <int MODE>
+template <int MODE, bool PRIME>
 __global__ void __launch_bounds__(512, 2)
     row_kernel(const __grid_constant__ MixPlan mp, const __grid_constant__ PassArgs a, int nl, int tpl, int nrows) {
   constexpr bool DM = MODE == ROW_DM_ITER;
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(512, 2)
 #pragma unroll 1
   for (int ph = INV ? 0 : 1; ph < 2; ph++) {  // ph 0: inverse, 1: forward
     const bool end = !UPD || ph == 1;
-    r = line_fft(r, r ? 0 : by, mp, L, tw, ph ? 1.0f : -1.0f, !UPD || ph == 0, end, load, store);
+    r = line_fft<PRIME>(r, r ? 0 : by, mp, L, tw, ph ? 1.0f : -1.0f, !UPD || ph == 0, end, load, store);
     if (end) break;
     if constexpr (UPD) {
       const float beta = iter_beta(a);
@@ -80,29 +80,39 @@ __global__ void __launch_bounds__(512, 2)
         }
       } else if (valid) {
         const UpdateRule rule = update_rule(a, beta);
-        for (int i0 = L.t; i0 < n; i0 += 4 * tpl) {
-          uint8_t f[4];
-          float2 g[4];
+        if (!rule.rare) {
+          for (int i0 = L.t; i0 < n; i0 += 4 * tpl) {
+            uint8_t f[4];
+            float2 g[4];
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int i = i0 + u * tpl;
-            f[u] = 0;
-            g[u] = zero;
-            if (i < n) {
-              f[u] = fl[i];
-              if (a.alg != ALG_ER) g[u] = g0[i];
+            for (int u = 0; u < 4; u++) {
+              const int i = i0 + u * tpl;
+              f[u] = i < n ? fl[i] : (uint8_t)0;
+              g[u] = i < n ? g0[i] : zero;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+              const int i = i0 + u * tpl, m = r + L.base + 8 * i;
+              if (i < n) {
+                const float2 w = packed::cmulw(at(m), a.inv_n, 0.0f);  // scale_cmul_dev
+                if (gp) gp[i] = w;
+                const float2 x = update_point(w, g[u], f[u], rule);
+                g1[i] = x;
+                at(m) = x;
+              }
             }
           }
-#pragma unroll
-          for (int u = 0; u < 4; u++) {
-            const int i = i0 + u * tpl, m = r + L.base + 8 * i;
-            if (i < n) {
-              const float2 w = packed::cmulw(at(m), a.inv_n, 0.0f);
-              if (gp) gp[i] = w;
-              const float2 x = rule.rare ? update_point_any(w, g[u], f[u], rule, a) : update_point(w, g[u], f[u], rule);
-              g1[i] = x;
-              at(m) = x;
-            }
+        } else {
+#pragma unroll 2
+          for (int i = L.t; i < n; i += tpl) {
+            const uint8_t f = fl[i];
+            const float2 g = a.alg != ALG_ER ? g0[i] : zero;
+            float2 &v = at(r + L.base + 8 * i);
+            const float2 w = scale_cmul_dev(v, a.inv_n);
+            if (gp) gp[i] = w;
+            const float2 x = update_point_any(w, g, f, rule, a);
+            g1[i] = x;
+            v = x;
           }
         }
       }
@@ -129,10 +139,11 @@ static cudaError_t launch_row(const LinePlan &px, const PassArgs &a, cudaStream_
   const int nl = (int)rows * PER;
   const size_t smem = smem_bytes(mp, nl);
   if (smem > kMixSmem) return cudaErrorNotSupported;
-  const cudaError_t e = ensure_smem<row_kernel<MODE>>(smem);
+  const dim3 grid((unsigned)((nrows + rows - 1) / rows)), block((nl * tpl + 31) / 32 * 32);
+  const cudaError_t e = mp.primes ? ensure_smem<row_kernel<MODE, true>>(smem) : ensure_smem<row_kernel<MODE, false>>(smem);
   if (e != cudaSuccess) return e;
-  return launch_maybe_pdl(row_kernel<MODE>, dim3((unsigned)((nrows + rows - 1) / rows)), dim3((nl * tpl + 31) / 32 * 32),
-                          smem, st, a.pdl != 0, mp, a, nl, tpl, (int)nrows);
+  return launch_maybe_pdl(mp.primes ? row_kernel<MODE, true> : row_kernel<MODE, false>, grid, block, smem, st, a.pdl != 0, mp,
+                          a, nl, tpl, (int)nrows);
 }
 
 }  // namespace mix
@@ -185,6 +196,8 @@ static bool make_mix_plan_as(MixPlan &mp, int n, const int *r, int ns, const flo
     st.nb = n / st.r;
     st.ns_magic = stride > 1 ? (unsigned)((0x100000000ull + stride - 1) / stride) : 0u;
     st.nb_magic = st.nb > 1 ? (unsigned)((0x100000000ull + st.nb - 1) / st.nb) : 0u;
+    const int groups = (st.nb + 1) / 2;  // prime_outputs
+    st.group_magic = groups > 1 ? (unsigned)((0x100000000ull + groups - 1) / groups) : 0u;
     st.tw1 = 8 * tws;
     tws += (r1 - 1) * stride;
     st.tw2 = 8 * tws;
@@ -197,6 +210,7 @@ static bool make_mix_plan_as(MixPlan &mp, int n, const int *r, int ns, const flo
     if (dout) mp.pitch = n + n / st.r;
     pad = dout;
     if (!st.kind) {
+      mp.primes = true;
       st.pw = pws;
       pws += r1;
       const int step = n / r1;

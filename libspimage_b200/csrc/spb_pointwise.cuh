@@ -201,15 +201,14 @@ __device__ __forceinline__ void project_many(float2 (&G)[U], const uint8_t (&f)[
 #pragma unroll
   for (int u = 0; u < U; u++) {
     if (FC && (a.constraints & C_CENTROSYM)) G[u].y = 0.0f;
-    s2[u] = packed::cabs2(G[u]);
+    s2[u] = fadd(fmul(G[u].y, G[u].y), fmul(G[u].x, G[u].x));
     fast = fast && (!(f[u] & FLAG_MEASURED) || sqrt_rn_nb_domain(s2[u]));
   }
   if (fast) {
 #pragma unroll
-    for (int u = 0; u < U; u += 2) {
-      const float2 m = div_sqrt_rn_nb2(make_float2(amp[u], amp[u + 1]), make_float2(s2[u], s2[u + 1]));
-      if (f[u] & FLAG_MEASURED) G[u] = packed::mul2(G[u], m.x);
-      if (f[u + 1] & FLAG_MEASURED) G[u + 1] = packed::mul2(G[u + 1], m.y);
+    for (int u = 0; u < U; u++) {
+      const float m = div_rn_nb(amp[u], sqrt_rn_nb(s2[u]));
+      if (f[u] & FLAG_MEASURED) G[u] = make_float2(fmul(G[u].x, m), fmul(G[u].y, m));
     }
   } else {
 #pragma unroll 1

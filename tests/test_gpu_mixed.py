@@ -84,3 +84,38 @@ def test_batch_of_ragged_frames(lib, oracle_mod):
         assert ref.iterate(14) == 0
         assert same_bits(gpu.start_model(b), ref.model()), b
     gpu.close()
+
+
+# the difference map's two projections in one launch: 8-point lines (256, 512)
+# and mixed-radix lines, with and without the Fourier constraint that only the
+# first of the two takes; 1024-point lines keep two launches
+@pytest.mark.parametrize("shape", [(256, 70), (512, 33), (45, 66), (1024, 24)])
+@pytest.mark.parametrize("cons,starts", [(2, 1), (16, 1), (1, 3)])
+def test_difference_map_projection_pair(lib, oracle_mod, shape, cons, starts):
+    from libspimage_b200 import synth
+
+    amp, mask, support, _ = synth.small_pattern(shape, seed=1)
+    seeds = list(range(5, 5 + starts))
+    gpu = lib.Phaser(shape)
+    gpu.set_algorithm(DIFFMAP, beta=0.8, constraints=cons)
+    gpu.start()
+    gpu.set_starts(starts)
+    gpu.set_amplitudes(amp, mask)
+    assert gpu.init_models(1, seeds) == 0
+    gpu.set_support(support)
+    assert gpu.iterate(1) == 0 and gpu.iterate(5) == 0
+    for b, seed in enumerate(seeds):
+        ref = setup(oracle_mod.Restatement(shape), shape, DIFFMAP, None, constraints=cons, beta=0.8, seed=seed)
+        assert ref.iterate(6) == 0
+        assert same_bits(gpu.start_model(b), ref.model()), b
+    gpu.close()
+
+
+# several waves of the projection pass: the instance with fewer registers
+@pytest.mark.parametrize("shape,alg", [((1024, 1536), RAAR), ((2048, 1024), HIO)])
+def test_projection_pass_of_several_waves(lib, oracle_mod, shape, alg):
+    ref, gpu = (setup(e, shape, alg, [(AREA, 4, 2.0, 0.1)]) for e in (oracle_mod.Restatement(shape, threads=8), lib.Phaser(shape)))
+    assert ref.iterate(6) == 0 and gpu.iterate(6) == 0
+    assert same_bits(gpu.model(), ref.model())
+    assert np.array_equal(gpu.flags(), ref.flags())
+    gpu.close()
