@@ -36,8 +36,9 @@ __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b)
 // Complex add and subtract as one packed f32x2 add (sm_100): each lane is
 // rounded exactly as __fadd_rn, and a - b is a + (-b) by IEEE definition, so
 // the bits equal the scalar recipe's while the instruction count halves.
-// Multiplies stay scalar: a packed product feeding a packed add is not kept
-// apart from it (measured: one-ulp differences), a scalar __fmul_rn is.
+// Multiplies stay scalar here: a packed multiply feeding a packed add is not
+// kept apart from it (measured: one-ulp differences), a scalar __fmul_rn is;
+// namespace packed below forms products that are.
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
 // (a.re*w.re - a.im*w.im, a.re*w.im + a.im*w.re), each product rounded

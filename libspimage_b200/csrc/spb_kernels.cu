@@ -21,7 +21,7 @@ namespace spb {
 
 // The general passes below (run-time stage loops) serve lines of one point and
 // lines without a plan in the mixed-radix kernels (make_mix_plan); every other
-// line runs in spb_fast.cu, spb_split.cu or spb_mixed_*.cu.
+// line runs in spb_fast*.cu, spb_split.cu or spb_mixed_*.cu.
 
 // ---------------------------------------------------------------- row pass
 template <int MODE>

@@ -1,5 +1,5 @@
 // Transforms of the pass kernels for every line length without a register kernel of its own
-// (spb_fast.cu, spb_split.cu): 2^a 3^b 5^c lengths that are not powers of
+// (spb_fast.cuh, spb_split.cu): 2^a 3^b 5^c lengths that are not powers of
 // two, and lengths with larger prime factors.
 //
 // Same transform as spb_fft.cuh, operation for operation: the canonical radix

@@ -1,4 +1,4 @@
-// Helpers shared by the register-resident pass kernels (spb_fast.cu: 16
+// Helpers shared by the register-resident pass kernels (spb_fast.cuh: 16
 // points per thread; spb_split.cu: 8 points per thread): asynchronous copies,
 // programmatic dependent launch, stage twiddles in shared memory, the
 // Fourier projection with its operands at hand, the layout of the

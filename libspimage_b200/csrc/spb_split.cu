@@ -1,5 +1,5 @@
 // Register-resident pass kernels with 8 points per thread, for patterns whose
-// lines are too few to fill the GPU with the 16-point kernels of spb_fast.cu
+// lines are too few to fill the GPU with the 16-point kernels of spb_fast.cuh
 // (a single 256x256 pattern has 256 lines per pass: 16 threads a line at 16
 // points each give less than one warp per SM, and the passes wait on
 // latency).  Here a line of N points is held by 2T threads (T = N/16 thread
@@ -27,7 +27,7 @@
 //  * radix 4 (four butterflies j per 16-point set): thread h holds the whole
 //    butterflies j = 2h, 2h+1.
 // Between stages the outputs go through the padded shared-memory line as in
-// spb_fast.cu.  Supported: N = 256, 512, 1024, 4096 (plans 16.16, 16.8.4,
+// spb_fast.cuh.  Supported: N = 256, 512, 1024, 4096 (plans 16.16, 16.8.4,
 // 16.16.4, 16.16.16), whose last stage leaves the outputs at M_h.
 //
 // Kernels: the row iteration pass (ROW_ITER: inverse x, update, forward x)
