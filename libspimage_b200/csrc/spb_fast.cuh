@@ -842,15 +842,6 @@ static bool row_tma_fits(const PassArgs &a) {
 }
 
 // ---------------------------------------------------------------- launch
-template <typename K>
-static cudaError_t set_smem(K k, size_t smem, bool &done) {
-  if (done) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) done = true;
-  return e;
-}
-
-
 template <int N, int MODE>
 static cudaError_t row_fast_launch(const LinePlan &px, const PassArgs &a, cudaStream_t st) {
   constexpr int T = N / 16;
@@ -929,15 +920,10 @@ static cudaError_t col_fast_launch_p(const LinePlan &pl, const PassArgs &a, cuda
     if (a.meas_words != proj_words(N)) return cudaErrorInvalidValue;
     smem += (size_t)C * amp_stride<N, C>() * sizeof(float) + (size_t)C * bits_stride<N, C>() * sizeof(uint32_t);
   }
-  auto k = col_fast_kernel<N, MODE, C, PREFETCH>;
-  static bool done = false;
-  static size_t done_smem = 0;
-  if (smem > done_smem) done = false;
-  cudaError_t e = set_smem(k, smem, done);
+  const cudaError_t e = ensure_smem<col_fast_kernel<N, MODE, C, PREFETCH>>(smem);
   if (e != cudaSuccess) return e;
-  if (smem > done_smem) done_smem = smem;
   dim3 grid((a.ncols + C - 1) / C, a.nouter);
-  return launch_maybe_pdl(k, grid, dim3(C * T), smem, st, a.pdl != 0, a, pl.stw);
+  return launch_maybe_pdl(col_fast_kernel<N, MODE, C, PREFETCH>, grid, dim3(C * T), smem, st, a.pdl != 0, a, pl.stw);
 }
 
 template <int N, int MODE>

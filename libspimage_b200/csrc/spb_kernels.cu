@@ -226,15 +226,6 @@ static int pow2_at_least(int v) {
   return p;
 }
 
-// dynamic shared memory attribute, set once per kernel and size
-template <typename K>
-static cudaError_t smem_attr(K k, size_t smem, size_t &done) {
-  if (smem <= done) return cudaSuccess;
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) done = smem;
-  return e;
-}
-
 template <int MODE>
 static cudaError_t row_launch(const LinePlan &px, const PassArgs &a, cudaStream_t st) {
   const int n = px.n;
@@ -246,12 +237,10 @@ static cudaError_t row_launch(const LinePlan &px, const PassArgs &a, cudaStream_
   constexpr bool UPD = (MODE == ROW_ITER || MODE == ROW_DM_ITER);
   // transform buffers, then (UPD) a slab of g0 and rpb*n bytes of flags
   const size_t smem = (size_t)(nbuf + (UPD ? 1 : 0)) * rpb * n * sizeof(float2) + (UPD ? (size_t)rpb * n : 0);
-  auto k = row_pass_kernel<MODE>;
-  static size_t done = 0;
-  cudaError_t e = smem_attr(k, smem, done);
+  const cudaError_t e = ensure_smem<row_pass_kernel<MODE>>(smem);
   if (e != cudaSuccess) return e;
   const long long grid = (nrows + rpb - 1) / rpb;
-  k<<<(unsigned)grid, rpb * tpr, smem, st>>>(px, a, tpr, rpb, nrows);
+  row_pass_kernel<MODE><<<(unsigned)grid, rpb * tpr, smem, st>>>(px, a, tpr, rpb, nrows);
   return cudaGetLastError();
 }
 
@@ -313,12 +302,10 @@ static cudaError_t col_launch(const LinePlan &pl, const PassArgs &a, cudaStream_
   if (tpc * ct < 32) tpc = 32 / ct;
   // two transform buffers, then (projection) n*ct amplitudes and n*ct flag bytes
   const size_t smem = (size_t)2 * n * ct * sizeof(float2) + (PROJ ? (size_t)n * ct * (sizeof(float) + 1) : 0);
-  auto k = col_pass_kernel<MODE>;
-  static size_t done = 0;
-  cudaError_t e = smem_attr(k, smem, done);
+  const cudaError_t e = ensure_smem<col_pass_kernel<MODE>>(smem);
   if (e != cudaSuccess) return e;
   dim3 grid((a.ncols + ct - 1) / ct, a.nouter);
-  k<<<grid, ct * tpc, smem, st>>>(pl, a, ct, tpc);
+  col_pass_kernel<MODE><<<grid, ct * tpc, smem, st>>>(pl, a, ct, tpc);
   return cudaGetLastError();
 }
 

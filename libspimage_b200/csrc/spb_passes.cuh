@@ -6,6 +6,9 @@
 #pragma once
 #include <math.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "spb_internal.h"
 #include "spb_pointwise.cuh"
 
@@ -118,13 +121,20 @@ inline cudaError_t device_sms(int *n) {
   return e;
 }
 
-// dynamic shared memory limit of kernel K raised to at least smem (once per size)
+// Dynamic shared memory limit of kernel K raised to at least smem.  One kernel
+// serves many line lengths, so host threads with contexts of different sizes
+// ask for different limits: the comparison, the call and the record are one
+// step under a lock, and the limit only grows (a launch that fits the recorded
+// limit takes no lock).
 template <auto K>
 static cudaError_t ensure_smem(size_t smem) {
-  static size_t have = 0;
-  if (smem <= have) return cudaSuccess;
+  static std::atomic<size_t> have{0};
+  static std::mutex lock;
+  if (smem <= have.load(std::memory_order_acquire)) return cudaSuccess;
+  std::lock_guard<std::mutex> hold(lock);
+  if (smem <= have.load(std::memory_order_relaxed)) return cudaSuccess;
   const cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) have = smem;
+  if (e == cudaSuccess) have.store(smem, std::memory_order_release);
   return e;
 }
 
