@@ -96,7 +96,11 @@ struct Axis {
   float2 *tw = nullptr;
 };
 
-int make_axis(Axis &ax, int n) {
+// The tables go up on the context's stream, and the copy is over on return: the
+// stream is a non-blocking one, so a copy on the legacy stream would not be
+// ordered before its first pass, and one from pageable memory may still be on
+// its way when that call returns.
+int make_axis(Axis &ax, int n, cudaStream_t stream) {
   int radix[64];
   const int ns = radix_plan(n, radix);
   if (ns > SPB_MAX_STAGES) return fail("axis length %d has too many radix stages", n);
@@ -129,7 +133,8 @@ int make_axis(Axis &ax, int n) {
     }
   h.insert(h.end(), st.begin(), st.end());
   CK(cudaMalloc(&ax.tw, sizeof(float2) * h.size()));
-  CK(cudaMemcpy(ax.tw, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(ax.tw, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice, stream));
+  CK(cudaStreamSynchronize(stream));  // h ends here
   ax.lp.tw = ax.tw;
   ax.lp.stw = ax.tw + n;
   for (MixPlan &mp : ax.mix) {
@@ -570,9 +575,9 @@ extern "C" int spb_ctx_create_batch(spb_ctx **out, int nx, int ny, int nz, int n
     if (cudaEventCreateWithFlags(&c->beta_ev[k], cudaEventDisableTiming) != cudaSuccess) rc = fail("cudaEventCreate");
     else if (cudaEventRecord(c->beta_ev[k], c->st) != cudaSuccess) rc = fail("cudaEventRecord");
   }
-  if (!rc && make_axis(c->ax, nx)) rc = -1;
-  if (!rc && make_axis(c->ay, ny)) rc = -1;
-  if (!rc && make_axis(c->az, nz)) rc = -1;
+  if (!rc && make_axis(c->ax, nx, c->st)) rc = -1;
+  if (!rc && make_axis(c->ay, ny, c->st)) rc = -1;
+  if (!rc && make_axis(c->az, nz, c->st)) rc = -1;
   if (!rc) {
     cudaMemsetAsync(c->amp, 0, nf1, c->st);
     cudaMemsetAsync(c->flags, 0, (size_t)c->ntot, c->st);
@@ -621,7 +626,7 @@ static int transform_ctx(spb_ctx **out, int nx, int ny, int nz, size_t bytes) {
     c->err_flag = (int *)carve(c, sizeof(int));
     if (cudaMemsetAsync(c->err_flag, 0, sizeof(int), c->st) != cudaSuccess) rc = fail("cudaMemsetAsync");
   }
-  if (!rc && (make_axis(c->ax, nx) || make_axis(c->ay, ny) || make_axis(c->az, nz))) rc = -1;
+  if (!rc && (make_axis(c->ax, nx, c->st) || make_axis(c->ay, ny, c->st) || make_axis(c->az, nz, c->st))) rc = -1;
   if (rc) {
     spb_ctx_destroy(c);
     return rc;

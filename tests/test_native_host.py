@@ -21,3 +21,10 @@ def run_native(tmp_path, name, *flags):
 def test_shared_memory_limit_never_falls(tmp_path):
     """Contexts of different line lengths on different host threads."""
     run_native(tmp_path, "smem_limit")
+
+
+def test_transform_tables_are_up_before_the_first_pass(tmp_path):
+    """A one-shot context's tables are not left on their way on another stream."""
+    lib = b.build()
+    fast = ["-O0", "-Xcicc", "-O0", "-Xptxas", "-O0", "-diag-suppress", "177"]  # nothing here runs on a device
+    run_native(tmp_path, "table_upload", *fast, lib, "-Xlinker", "-rpath=" + os.path.dirname(lib))
