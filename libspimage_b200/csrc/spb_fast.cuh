@@ -842,6 +842,19 @@ static bool row_tma_fits(const PassArgs &a) {
 }
 
 // ---------------------------------------------------------------- launch
+// LPB rows a block, g0 fetched between the transforms
+template <int N, int MODE>
+static cudaError_t row_late_launch(const LinePlan &px, const PassArgs &a, int LPB, size_t smem, cudaStream_t st) {
+  const cudaError_t e = ensure_smem<row_fast_kernel<N, MODE, true>>(smem);
+  if (e != cudaSuccess) return e;
+  const long long nrows = a.n / N;
+  return launch_maybe_pdl(row_fast_kernel<N, MODE, true>, dim3((unsigned)((nrows + LPB - 1) / LPB)), dim3(LPB * (N / 16)),
+                          smem, st, a.pdl != 0, a, px.stw, (int)nrows);
+}
+// the same for ROW_ITER and N = 128 and 256 (spb_fast_rows_late.cu)
+template <int N>
+cudaError_t row_iter_late(const LinePlan &px, const PassArgs &a, int LPB, size_t smem, cudaStream_t st);
+
 template <int N, int MODE>
 static cudaError_t row_fast_launch(const LinePlan &px, const PassArgs &a, cudaStream_t st) {
   constexpr int T = N / 16;
@@ -890,11 +903,10 @@ static cudaError_t row_fast_launch(const LinePlan &px, const PassArgs &a, cudaSt
                                 a.pdl != 0, a, px.stw, (int)nrows);
       }
     }
-    if (late) {
-      cudaError_t e = ensure_smem<row_fast_kernel<N, MODE, true>>(smem_late);
-      if (e != cudaSuccess) return e;
-      return launch_maybe_pdl(row_fast_kernel<N, MODE, true>, dim3((unsigned)grid), dim3(LPB * T), smem_late, st,
-                              a.pdl != 0, a, px.stw, (int)nrows);
+    if constexpr (MODE == ROW_ITER && (N == 128 || N == 256)) {
+      if (late) return row_iter_late<N>(px, a, LPB, smem_late, st);
+    } else if (late) {
+      return row_late_launch<N, MODE>(px, a, LPB, smem_late, st);
     }
     cudaError_t e = ensure_smem<row_fast_kernel<N, MODE, false>>(smem_early);
     if (e != cudaSuccess) return e;
