@@ -138,7 +138,7 @@ constexpr size_t kMixSmem = 227 * 1024;  // dynamic shared memory a block may ta
 struct MixStep {
   int kind, r;              // r: points of a composite butterfly
   int ns, nb;               // points between its outputs; butterflies per line (n / r)
-  unsigned ns_magic, nb_magic, group_magic;  // quotients by ns, nb and (nb + 1) / 2 as a high product (unused for 1)
+  unsigned ns_magic, nb_magic;  // quotients by ns and nb as a high product (unused for 1)
   int tw1, tw2, pw;         // its tables: byte offsets in the stage table (first, second stage), entry of the prime tables
   int din;                  // free elements after every ns points of its input
   int sin, qout;            // elements between a butterfly's inputs, between the outputs of q and q + 1

@@ -33,9 +33,9 @@
 // the steps (load, butterfly, store, barrier), larger ones by instruction
 // issue (55-59 % issue active at 192^3 before the pointwise loops were made
 // branch-free).  Per iteration slot, the run-time stage loops these kernels
-// replaced / these kernels: HIO 600^2 38 / 21 us, 768^2 51 / 30, 1200^2 96 / 54,
-// 100^3 85 / 48, 192^3 386 / 188, 384^3 3545 / 1910, 1000^2 39.0 / 36.4 (a
-// compile-time plan before), RAAR 650x670 (2.5.5.13 x 2.5.67) 1818 / 57,
+// replaced / these kernels: HIO 600^2 38 / 22 us, 768^2 51 / 28.5, 1200^2 95 / 54.5,
+// 100^3 83 / 48.5, 192^3 384 / 187, 384^3 3270 / 1858, 1000^2 39.0 / 37.3 (a
+// compile-time plan before), RAAR 650x670 (2.5.5.13 x 2.5.67) 1816 / 57,
 // 257x263 49000 / 80.  Two lines a thread (shared index arithmetic and
 // twiddle loads, 128 registers) was slower everywhere: 1000^2 39.6 against
 // 36.0, 8 x 384^2 57.5 against 44.9.
@@ -243,8 +243,9 @@ __device__ __forceinline__ void prime_outputs(int x, int y, const Lay &L, const 
                                               const MixStep &s, const Dir &g, bool last, Store store) {
   const int R = s.r, ns = s.ns, nb = s.nb, sin = s.sin * L.es;
   const int groups = (nb + JB - 1) / JB, half = (R + 1) / 2;
+  const unsigned group_magic = 0xffffffffu / groups + 1;  // quotients by groups > 1 as a high product
   for (int t = L.t; t < groups * half; t += L.tpl) {
-    const int m = groups == 1 ? t : (int)__umulhi((unsigned)t, s.group_magic);
+    const int m = groups == 1 ? t : (int)__umulhi((unsigned)t, group_magic);
     const int b0 = t - m * groups;
     int in[JB], out[JB];
     float2 u[JB], v[JB];
@@ -297,8 +298,8 @@ __device__ __forceinline__ void prime_outputs(int x, int y, const Lay &L, const 
 }
 
 // A prime stage R >= 7: its inputs take their twiddles in place, once, then
-// prime_outputs.
-template <class Load, class Store>
+// its outputs are formed.
+template <int PRIMES, class Load, class Store>
 __device__ __forceinline__ void stage_prime(int x, int y, const Lay &L, int tw, const float2 *__restrict__ wr,
                                             const MixStep &s, const Dir &g, bool first, bool last, Load load,
                                             Store store) {
@@ -324,17 +325,58 @@ __device__ __forceinline__ void stage_prime(int x, int y, const Lay &L, int tw, 
     }
     __syncthreads();
   }
-  if (nb > 1) prime_outputs<2>(x, y, L, wr, s, g, last, store);
-  else prime_outputs<1>(x, y, L, wr, s, g, last, store);
+  if constexpr (PRIMES == 2) {
+    if (nb > 1) prime_outputs<2>(x, y, L, wr, s, g, last, store);
+    else prime_outputs<1>(x, y, L, wr, s, g, last, store);
+  } else {  // one butterfly a task, a plainer loop (line_fft)
+    const int half = (R + 1) / 2;
+    for (int t = L.t; t < nb * half; t += L.tpl) {
+      const int m = nb == 1 ? t : (int)__umulhi((unsigned)t, s.nb_magic);
+      const int b = t - m * nb;
+      const int q0 = ns == 1 ? b : (int)__umulhi((unsigned)b, s.ns_magic);
+      int in = x + (b + q0 * s.din) * L.es;
+      const int out = b + q0 * ns * (R - 1);  // point of output 0
+      const float2 a0 = at(in);
+      float2 u = a0, v = a0;
+      if (m == 0) {
+#pragma unroll 4
+        for (int q = 1; q < R; q++) u = cadd(u, at(in += sin));
+      } else {
+        int e = 0;
+#pragma unroll 4
+        for (int q = 1; q < R; q++) {
+          e += m;
+          e = e >= R ? e - R : e;
+          const float2 w = __ldg(wr + e), aq = at(in += sin);
+          const float2 p = mul(aq, w.x, g), h = mul(swp(aq), w.y, g);
+          u = cadd(u, __ffma2_rn(h, neg(g.w), p));
+          v = cadd(v, __ffma2_rn(h, g.w, p));
+        }
+      }
+      const int ou = out + m * ns, ov = out + (R - m) * ns;
+      if (last) {
+        store(ou, u);
+        if (m) store(ov, v);
+      } else {
+        at(y + ou * L.es) = u;
+        if (m) at(y + ov * L.es) = v;
+      }
+    }
+  }
 }
 
 // Every stage of the block's lines, from the buffer at x (or, with from_mem,
 // from load()) to a buffer, or with to_mem to store(); returns the buffer (x
 // or y) of the result.  All threads call it; it synchronises after every step
-// that ends in shared memory.  tw: where the stage tables start.  PRIME: the
-// plan has prime steps (kernels of plans without any leave their code out, for
-// its registers: HIO 600^2 22.3 -> 21.5 us per slot).
-template <bool PRIME, class Load, class Store>
+// that ends in shared memory.  tw: where the stage tables start.  PRIMES: 2
+// for plans with prime steps; the kernels of plans without any leave them out
+// (0), except for the columns' forward and inverse passes (1): no plan of theirs
+// reaches the plain loop either, but without it the compiler allocates their 64
+// registers worse (24 + 48 bytes of spill stores and loads in the projection,
+// 12 + 16 with it).  Projection and blur without / with, us a pass at 192^3: 76.0 /
+// 71.5 and 57.6 / 53.6; in the passes of one transform it costs (192^3, one
+// direction 39.5 / 40.2, |blur| rows 31.1 / 32.5).
+template <int PRIMES, class Load, class Store>
 __device__ __forceinline__ int line_fft(int x, int y, const MixPlan &mp, const Lay &L, int tw, float d, bool from_mem,
                                          bool to_mem, Load load, Store store) {
   const Dir g = make_dir(d, mp.neg0);
@@ -348,7 +390,7 @@ __device__ __forceinline__ int line_fft(int x, int y, const MixPlan &mp, const L
     switch (s.kind) {
       SPB_MIX_KINDS(SPB_MIX_STEP)
       default:
-        if constexpr (PRIME) stage_prime(x, y, L, tw, mp.pw + s.pw, s, g, first, last, load, store);
+        if constexpr (PRIMES != 0) stage_prime<PRIMES>(x, y, L, tw, mp.pw + s.pw, s, g, first, last, load, store);
         break;
     }
 #undef SPB_MIX_STEP

@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(512, 2)
 #pragma unroll 1
   for (int ph = FWD ? 0 : 1; ph < 2; ph++) {  // ph 0: forward, 1: inverse
     const bool end = !MID || ph == 1;
-    r = line_fft<PRIME>(r, r ? 0 : by, mp, L, tw, ph ? -1.0f : 1.0f, !MID || ph == 0, end, load, store);
+    r = line_fft<PRIME ? 2 : MID>(r, r ? 0 : by, mp, L, tw, ph ? -1.0f : 1.0f, !MID || ph == 0, end, load, store);
     if (end) break;
     if constexpr (PROJ) {
       const long long ai0 = base % a.n_start;  // the amplitude side holds one start
