@@ -21,7 +21,7 @@ INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libspimage_b200.so")
 
-CU_SOURCES = ["spb_kernels.cu", "spb_fast.cu", "spb_fast_rows_cols_long.cu", "spb_fast_rows_late.cu", "spb_fast_cols_short.cu", "spb_split.cu", "spb_mixed_rows.cu", "spb_mixed_cols.cu", "spb_capi.cu"]
+CU_SOURCES = ["spb_kernels.cu", "spb_fast.cu", "spb_fast_rows_cols_long.cu", "spb_fast_rows_late.cu", "spb_fast_cols_short.cu", "spb_ct.cu", "spb_split.cu", "spb_mixed_rows.cu", "spb_mixed_cols.cu", "spb_capi.cu"]
 C_SOURCES = ["host/image.c", "host/phasing.c", "host/support_update.c", "host/fft.c", "host/prtf.c"]
 CXX_SOURCES = ["host/serve.cpp"]
 HEADERS = ["spb_fft.cuh", "spb_internal.h", "spb_pointwise.cuh", "spb_passes.cuh", "spb_mixed.cuh", "spb_fast.cuh", "host/host_internal.h"]

@@ -156,6 +156,12 @@ struct MixPlan {
 bool make_mix_plan(MixPlan &mp, int n, const int *radix, int nstages, const float2 *tw, bool pairs);
 cudaError_t launch_row_mixed(int mode, const LinePlan &px, const PassArgs &a, cudaStream_t st);
 cudaError_t launch_col_mixed(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st);
+// passes with compile-time plans (spb_ct.cu) for the grids of 192, 384 and
+// 1000-point lines where they are the faster ones; else cudaErrorNotSupported
+cudaError_t launch_row_ct(int mode, const LinePlan &px, const PassArgs &a, cudaStream_t st);
+cudaError_t launch_col_ct(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st);
+// whether a column pass of so many lines of n points runs there
+bool ct_columns(int mode, int n, long long lines, const PassArgs &a);
 
 // register-resident kernels (spb_fast.cu); cudaErrorNotSupported when the
 // line length or mode has none

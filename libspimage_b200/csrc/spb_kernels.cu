@@ -21,7 +21,7 @@ namespace spb {
 
 // The general passes below (run-time stage loops) serve lines of one point and
 // lines without a plan in the mixed-radix kernels (make_mix_plan); every other
-// line runs in spb_fast*.cu, spb_split.cu or spb_mixed_*.cu.
+// line runs in spb_fast*.cu, spb_split.cu, spb_ct.cu or spb_mixed_*.cu.
 
 // ---------------------------------------------------------------- row pass
 template <int MODE>
@@ -266,6 +266,8 @@ cudaError_t launch_row(int mode, const LinePlan &px, const PassArgs &a, cudaStre
   }
   const cudaError_t fe = launch_row_fast(mode, px, a, st);
   if (fe != cudaErrorNotSupported) return fe;
+  const cudaError_t ce = launch_row_ct(mode, px, a, st);
+  if (ce != cudaErrorNotSupported) return ce;
   const cudaError_t me = launch_row_mixed(mode, px, a, st);
   if (me != cudaErrorNotSupported) return me;
   switch (mode) {
@@ -324,10 +326,16 @@ cudaError_t launch_col(int mode, const LinePlan &pl, int line_len, const PassArg
       if (se != cudaErrorNotSupported) return se;
     }
     if ((pl.n & (pl.n - 1)) == 0) return cudaErrorNotSupported;
+    // two launches with a compile-time plan beat one without at 1000 points (DM
+    // 1000^2 x 8 508 -> 476 us per slot), not at 192 and 384 (192^2 x 1 15.2 -> 18.6,
+    // 384^2 x 4 44.5 -> 48.8)
+    if (pl.n == 1000 && ct_columns(COL_PROJECT, pl.n, (long long)a.ncols * a.nouter, a)) return cudaErrorNotSupported;
     return launch_col_mixed(mode, pl, a, st);
   }
   const cudaError_t fe = launch_col_fast(mode, pl, a, st);
   if (fe != cudaErrorNotSupported) return fe;
+  const cudaError_t ce = launch_col_ct(mode, pl, a, st);
+  if (ce != cudaErrorNotSupported) return ce;
   const cudaError_t me = launch_col_mixed(mode, pl, a, st);
   if (me != cudaErrorNotSupported) return me;
   switch (mode) {
