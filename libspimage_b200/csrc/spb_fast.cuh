@@ -704,20 +704,23 @@ static cudaError_t col_tma_launch(const LinePlan &pl, const PassArgs &a, cudaStr
     return cudaErrorNotSupported;
   dim3 grid((a.ncols + C - 1) / C, a.nouter);
   cudaError_t e = ensure_smem<col_tma_kernel<N, MODE, C, false>>(smem);
-  int per_sm = 0, many = 0, nsm = 0;
-  if (e == cudaSuccess) e = device_sms(&nsm);
-  if (e == cudaSuccess)
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, col_tma_kernel<N, MODE, C, false>, C * T, smem);
-  // several waves, and more blocks an SM with fewer registers: RAAR 2048^2 76 ->
-  // 68 us, 8 x 1024^2 122 -> 110 us per slot (two -> three blocks of 256 threads)
-  if (e == cudaSuccess && (long long)grid.x * grid.y > (long long)per_sm * nsm) {
-    e = ensure_smem<col_tma_kernel<N, MODE, C, true>>(smem);
+  if constexpr (MODE != COL_BLUR && (N == 256 || N >= 1024)) {
+    // several waves, and more blocks an SM with fewer registers: RAAR 2048^2 76 ->
+    // 68 us, 8 x 1024^2 122 -> 110 us per slot (two -> three blocks of 256 threads).
+    // The other lengths and the blur take 80 registers or fewer as they are.
+    int per_sm = 0, many = 0, nsm = 0;
+    if (e == cudaSuccess) e = device_sms(&nsm);
     if (e == cudaSuccess)
-      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&many, col_tma_kernel<N, MODE, C, true>, C * T, smem);
+      e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, col_tma_kernel<N, MODE, C, false>, C * T, smem);
+    if (e == cudaSuccess && (long long)grid.x * grid.y > (long long)per_sm * nsm) {
+      e = ensure_smem<col_tma_kernel<N, MODE, C, true>>(smem);
+      if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&many, col_tma_kernel<N, MODE, C, true>, C * T, smem);
+    }
+    if (e == cudaSuccess && many > per_sm)
+      return launch_maybe_pdl(col_tma_kernel<N, MODE, C, true>, grid, dim3(C * T), smem, st, a.pdl != 0, a, pl.stw, tin, tout);
   }
   if (e != cudaSuccess) return e;
-  if (many > per_sm)
-    return launch_maybe_pdl(col_tma_kernel<N, MODE, C, true>, grid, dim3(C * T), smem, st, a.pdl != 0, a, pl.stw, tin, tout);
   return launch_maybe_pdl(col_tma_kernel<N, MODE, C, false>, grid, dim3(C * T), smem, st, a.pdl != 0, a, pl.stw, tin, tout);
 }
 
