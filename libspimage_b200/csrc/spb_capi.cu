@@ -599,7 +599,8 @@ extern "C" int spb_ctx_create_batch(spb_ctx **out, int nx, int ny, int nz, int n
 // spb_prtf_host): a stream, the transforms' tables and one allocation of `bytes`
 // that carve() shares out, instead of the phasing state's 17 allocations, its
 // pinned rings and 130 events, which took longer than the transforms
-// themselves (an FFT of 900x1200: 10.3 ms a call, 0.1 of it on the GPU).
+// themselves (a call's median on one box, its host noisy: FFT of 900x1200 10.6-13 ->
+// 2.6 ms, 0.1 of it on the GPU; PRTF of 8 x 256^2 7.8 -> 3.6 ms).
 const size_t kCarveAlign = 256;
 static size_t carved(size_t bytes) { return (bytes + kCarveAlign - 1) / kCarveAlign * kCarveAlign; }
 static void *carve(spb_ctx *c, size_t bytes) {

@@ -349,7 +349,7 @@ cudaError_t check_roundings(unsigned lo, unsigned hi, unsigned long long ndiv, u
 // Columns per block the projection pass offers besides the built-in width:
 // lines of 256, 512 and 1024 points, C a power of two with C*N/16 <= 256
 // threads and C <= 16 (the shared-memory skew is 16/C words); and the
-// lengths the general kernels run with compile-time plans (general_col_width_ok).
+// lengths 192, 384 and 1000 (general_col_width_ok).
 bool col_width_ok(int n, int w) {
   if (w < 1 || w > 16 || (w & (w - 1))) return false;
   if (n != 256 && n != 512 && n != 1024) return general_col_width_ok(n, w);

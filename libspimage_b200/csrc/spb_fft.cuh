@@ -180,9 +180,11 @@ __device__ __forceinline__ void bf5(float2 *a) {
 // it is contracted with the packed add that follows (measured: one-ulp
 // differences in 31 % of twiddle products; none in 2^28 with this form).  The
 // -0 sits in constant memory so that the compiler cannot fold it away.  The
-// packed forms take 10-30 registers more (pairs for the constants), so kernels
-// that live on their occupancy keep the forms above: used in packed form, the
-// row pass of 64 starts of 512^2 went from 111 to 118 us.
+// packed forms take 10-30 registers more (pairs for the constants).  The 16-point
+// passes keep the forms above: in packed form the row pass of 64 starts of 512^2
+// went from 111 to 118 us.  The persistent kernels use them although they spill
+// more at their 64 registers (148-172 bytes, 16-64 before): 256 starts of 64^2 17.5 ->
+// 15.8 us per slot.
 namespace packed {
 static __constant__ float2 kNeg0 = {-0.0f, -0.0f};
 __device__ __forceinline__ float2 cswap(float2 a) { return make_float2(a.y, a.x); }

@@ -80,7 +80,7 @@ struct PassArgs {
   int split;
   // columns per block of the projection pass (0: the built-in width); see col_width_ok
   int col_width;
-  // projection pass column tiles by TMA (spb_fast.cu col_tma_kernel): 2 always where the
+  // projection pass column tiles by TMA (spb_fast.cuh col_tma_kernel): 2 always where the
   // tile fits, 0 where it fits at the built-in width, 1 never
   int tma;
   int *err_flag;  // set by a kernel that could not do its work (device): 1 a bounded wait ran out, 2 a misaligned TMA tile
@@ -122,7 +122,7 @@ struct SelectState {
 };
 static_assert(sizeof(SelectState) == 8216, "the selection state keeps its size");
 
-// Steps of a line transform in the mixed-radix kernels (spb_mixed.cu): one
+// Steps of a line transform in the mixed-radix kernels (spb_mixed.cuh): one
 // stage of the canonical plan, or two short consecutive ones run as one.
 // Radices with a kernel, and the pairs that have one; other radices (primes
 // from 7) are kind 0.  n * (the largest index a magic divides) stays below 2^32.
@@ -146,7 +146,7 @@ struct MixStep {
 struct MixPlan {
   int n, nsteps, pitch;  // pitch: elements of a line's buffer
   bool primes;           // some step is a prime
-  float neg0;            // -0 (see spb_mixed.cu)
+  float neg0;            // -0 (see spb_mixed.cuh)
   const float2 *stw;     // stage tables (LinePlan::stw)
   const float2 *pw;      // per prime step: W_R^e, e < R (device)
   MixStep step[kMixMaxSteps];
@@ -163,13 +163,13 @@ cudaError_t launch_col_ct(int mode, const LinePlan &pl, const PassArgs &a, cudaS
 // whether a column pass of so many lines of n points runs there
 bool ct_columns(int mode, int n, long long lines, const PassArgs &a);
 
-// register-resident kernels (spb_fast.cu); cudaErrorNotSupported when the
+// register-resident kernels (spb_fast.cuh); cudaErrorNotSupported when the
 // line length or mode has none
 cudaError_t launch_row_fast(int mode, const LinePlan &px, const PassArgs &a, cudaStream_t st);
 cudaError_t launch_col_fast(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st);
 // whether the projection pass has a kernel of w columns per block for lines of n points
 bool col_width_ok(int n, int w);
-// the same for mixed-radix lines (192, 384 and 1000 points)
+// the same for lines of 192, 384 and 1000 points
 bool general_col_width_ok(int n, int w);
 // all iterations of a call for every start of an N x N pattern (N = 32, 64,
 // 128), one block per start with its spectrum resident (spb_fast.cu); a.dst
@@ -187,8 +187,8 @@ cudaError_t launch_gauss_table(const PassArgs &a, float *tab, cudaStream_t st);
 cudaError_t check_roundings(unsigned lo, unsigned hi, unsigned long long ndiv, unsigned long long seed,
                             unsigned a_stride, unsigned long long *d_bad);
 
-// host-side launchers (spb_kernels.cu): register kernels where available,
-// general kernels otherwise
+// host-side launchers (spb_kernels.cu): the register kernels, the ones with
+// compile-time plans, the mixed-radix or the general ones, whichever takes the pass first
 cudaError_t launch_row(int mode, const LinePlan &px, const PassArgs &a, cudaStream_t st);
 cudaError_t launch_col(int mode, const LinePlan &pl, int line_len, const PassArgs &a, cudaStream_t st);
 // support selection and reductions; nb starts of n pixels each, start b at offset b*n

@@ -463,7 +463,8 @@ inline int threads_per_line(const MixPlan &mp, long long lines, int most) {
 }
 
 // Stages run as one save an exchange but leave fewer, longer tasks: not where
-// their tasks do not give the SMs two warps each (192^2: 14.8 -> 12.5 us).
+// their tasks do not give the SMs two warps each (120^2 13.8 -> 12.0 us per slot,
+// 240^2 17.5 -> 13.9).
 inline const MixPlan &choose_plan(const LinePlan &pl, long long lines) {
   return pl.mix[lines * most_tasks(pl.mix[0]) < 64LL * num_sms() ? 1 : 0];
 }

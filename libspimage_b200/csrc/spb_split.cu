@@ -489,7 +489,7 @@ cudaError_t launch_row_split(int mode, const LinePlan &px, const PassArgs &a, cu
 }
 
 cudaError_t launch_col_split(int mode, const LinePlan &pl, const PassArgs &a, cudaStream_t st) {
-  if (pl.stw && mode == COL_PROJECT_PAIR) {  // the lengths the built-in choice runs here
+  if (pl.stw && mode == COL_PROJECT_PAIR) {  // other 8-point lengths keep two launches
     if (pl.n == 256) return col_split_launch<256, COL_PROJECT_PAIR>(pl, a, st);
     if (pl.n == 512) return col_split_launch<512, COL_PROJECT_PAIR>(pl, a, st);
   }
